@@ -20,6 +20,7 @@
 // traversal.  Closest hit: smallest t, ties to the lowest (instance,
 // primitive); t is the refined plane-equation distance in the winning
 // instance's object space.
+#include "bvh2.cuh"
 #include "common.cuh"
 #include "lbvh.cuh"
 #include "rtmath.cuh"
@@ -109,69 +110,192 @@ __device__ __forceinline__ void ray_to_object(const float *w, const Ray &W, Ray 
   ray_setup(make_float4(ro[0], ro[1], ro[2], W.tmin), make_float4(rd[0], rd[1], rd[2], W.tmax), O);
 }
 
-struct InstMeshes {
-  const uint32_t *tri_off;  // null: one mesh of n_all triangles
-  uint32_t meshes, n_all;
+struct InstArgs {
+  const Bvh2Node *tnodes;  // top level
+  const uint32_t *tids;
+  uint32_t ninst;
+  const float *troot;
+  const InstanceRec *inst;
+  const float *w2o;
+  const Bvh2Node *nodes;  // bottom level
+  const float4 *leaf;
+  const uint32_t *tri_off;  // null: one mesh of n triangles
+  uint32_t meshes, n;
+  const float4 *rays;
+  uint64_t nrays;
+  uint32_t ray_mask;
+  Hit *hits;
+  uint32_t *hit_inst;
+  unsigned long long *counter;
+  uint32_t *err;
 };
 
 constexpr int kInstThreads = 128;
-constexpr int kInstStack = 64;
+constexpr int kInstWarps = kInstThreads / 32;
+constexpr int kInstShared = 10;  // stack entries in shared memory
+constexpr int kInstDepth = 128;  // 62 levels of each tree
 constexpr int kInstRefill = 4;
+constexpr int kInstEnter = 8;
+constexpr int kInstSteps = 6;
+constexpr int kInstFlush = 12;
+constexpr int kInstQueue = 96;  // a step queues at most 64
+constexpr int kInstCtas = 8;
+constexpr int kWalkLeave = kWalkEnd + 1;  // below a mesh's entries: back to the top level
 
-// One lane per ray from a global counter, warp-uniform visit loop; lanes
-// whose rays finished take new rays once kInstRefill of the 32 are idle
-// (16,384 instances, 16.8M rays: 32 rays per warp without refill 147 ms,
-// refill at 16 / 8 / 4 idle lanes 119.6 / 109.5 / 105.7 ms).  The top-level stack holds references (inner node >= 0, leaf
-// ~slot) with their entry distances, so a popped reference behind the best hit
-// is dropped; the bottom-level stack holds node indices.
-template <bool ANY>
-__global__ void __launch_bounds__(kInstThreads) k_trace_inst(const Bvh2Node *tnodes, const uint32_t *tids, uint32_t ninst,
-                                                             const float *troot, const InstanceRec *inst,
-                                                             const float *w2o, const Bvh2Node *blas_all,
-                                                             const float4 *leaf_all, InstMeshes im, const float4 *rays,
-                                                             uint64_t nrays, uint32_t ray_mask, Hit *hits,
-                                                             uint32_t *hit_inst, unsigned long long *counter,
-                                                             uint32_t *err) {
+// Finished rays that hit something, refined 32 at a time.
+struct InstRefineQueue {
+  unsigned long long ray[64];
+  uint32_t inst[64], slot[64];
+};
+
+// t of the winner on its object-space ray, recomputed from the ray (the same
+// operations, so the same bits as during the walk).
+__device__ __forceinline__ void inst_refine(const InstArgs &A, const InstRefineQueue &q, int first, int count) {
   const int lane = threadIdx.x & 31;
-  const uint32_t lt = (1u << lane) - 1u;
-  bool active = false, drained = false, done = true;
-  uint64_t r = 0;
-  Ray W, O;
-  uint32_t best = kMiss, binst = kMiss, bslot = 0;
-  float bt = 0.0f;
-  int tref[kInstStack];
-  float ttn[kInstStack];
-  int tsp = 0;
-  int bstack[kInstStack];
-  int bsp = 0;
-  int level = 0, cur = 0, bnode = 0;
-  uint32_t ci = 0;  // instance being walked
-  const Bvh2Node *bvh = blas_all;
-  const float4 *leaf = leaf_all;
-  auto tri_test = [&](uint32_t slot) {
-    const float4 a = __ldg(leaf + 3 * (size_t)slot), b = __ldg(leaf + 3 * (size_t)slot + 1),
-                 c = __ldg(leaf + 3 * (size_t)slot + 2);
+  __syncwarp();
+  if (lane < count) {
+    const unsigned long long r = q.ray[first + lane];
+    const uint32_t inst = q.inst[first + lane], slot = q.slot[first + lane];
+    const float4 o = __ldg(A.rays + 2 * r), d = __ldg(A.rays + 2 * r + 1);
+    Ray W, O;
+    W.ox = o.x; W.oy = o.y; W.oz = o.z; W.tmin = o.w;
+    W.dx = d.x; W.dy = d.y; W.dz = d.z; W.tmax = d.w;
+    ray_to_object(A.w2o + 12 * (size_t)inst, W, O);
+    const float4 a = __ldg(A.leaf + 3 * (size_t)slot), b = __ldg(A.leaf + 3 * (size_t)slot + 1),
+                 c = __ldg(A.leaf + 3 * (size_t)slot + 2);
     const float v0[3] = {a.x, a.y, a.z}, v1[3] = {b.x, b.y, b.z}, v2[3] = {c.x, c.y, c.z};
-    const uint32_t id = __float_as_uint(a.w);
-    float t;
-    if (isect_tri(O, v0, v1, v2, t) &&
-        (best == kMiss || t < bt || (t == bt && (ci < binst || (ci == binst && id < best))))) {
-      best = id;
-      binst = ci;
-      bslot = slot;
+    Hit h;
+    h.prim = __float_as_uint(a.w);
+    h.t = refine_t(O, v0, v1, v2);
+    A.hits[r] = h;
+    if (A.hit_inst) A.hit_inst[r] = inst;
+  }
+  __syncwarp();
+}
+
+// One lane per ray from a global counter.  A lane walks the top level with
+// its world ray; an instance it reaches waits until kInstEnter lanes of the
+// warp want to enter one (or no lane can do anything else), then these map
+// their rays into object space together -- two divisions, four reciprocals
+// and twelve loads that a lane alone would keep the warp waiting for -- and
+// walk that mesh on the same stack, above a mark that leads back to the top
+// level.  Closest hit queues its triangle tests per warp and runs them with all
+// lanes (as the one-level traversal does); the queue is emptied before a lane
+// with tests in it enters another instance, so the tests of a lane all belong
+// to the instance it entered last, whose object-space ray is in shared memory.
+// With entries, node steps and tests of single lanes each taking the whole
+// warp's time, 7.6 of 32 lanes were active; now 19 are, and the L1 data pipe
+// (76 % busy, see load_child) and load latency bound it.  4.2 M rays over
+// 16,384 instances: 18.0 -> 10.8 ms.  Entering at 1 / 4 / 6 / 8 / 12 waiting
+// lanes: 12.8 / 12.3 / 10.8 / 10.8 / 11.1 ms (the first two before the CTAs
+// per SM went from 6 to 8, 12.1 -> 10.8 ms); 2 / 4 / 6 / 8 node steps between
+// two looks at entries, flush and refill: 12.5 / 12.1 / 11.2 / 12.0 ms then.
+// 10 stack entries in shared memory against 8 and 6: 10.8 / 11.2 / 11.5 ms.
+template <bool ANY, bool V8>
+__global__ void __launch_bounds__(kInstThreads, kInstCtas) k_trace_inst(const InstArgs A) {
+  __shared__ float2 s_stack[kInstShared][kInstThreads];
+  __shared__ InstRefineQueue s_rq[kInstWarps];
+  __shared__ uint32_t s_qslot[kInstWarps][kInstQueue];
+  __shared__ uint8_t s_qlane[kInstWarps][kInstQueue];
+  __shared__ unsigned long long s_key[kInstWarps][32];  // closest (t, id) of the tests since the last merge
+  __shared__ uint32_t s_kslot[kInstWarps][32];
+  __shared__ float s_obj[7][kInstThreads];    // origin, Sx, Sy, Sz; tmax
+  __shared__ int s_objk[kInstThreads];        // kx | ky << 2 | kz << 4
+  __shared__ uint32_t s_best[2][kInstThreads];  // instance and leaf slot of the best hit
+  __shared__ unsigned long long s_rid[kInstThreads];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, wbase = tid & ~31;
+  const uint32_t lt = (1u << lane) - 1u;
+  InstRefineQueue &rq = s_rq[w];
+  uint32_t *qslot = s_qslot[w];
+  uint8_t *qlane = s_qlane[w];
+  const float kNone = __int_as_float(0x7fffffff);
+  bool active = false, drained = false, pending = false, inside = false;
+  RayPairs P;
+  P.nxy = P.nzz = P.ixy = P.izz = 0;
+  P.tmin = 0.0f;
+  float bt = 0.0f;
+  uint32_t ci = 0, base_leaf = 0, base_node = 0;  // the instance entered last, its mesh's arrays
+  int nq = 0, nrq = 0;
+  Walk W;
+  W.start();
+  W.node = kWalkEnd;
+  float2 *const sh = &s_stack[0][tid];
+  float2 over[kInstDepth - kInstShared];
+
+  // one triangle of lane o's object-space ray
+  auto tri_test = [&](uint32_t slot, int o, float tmin, uint32_t &id, float &t) -> bool {
+    Ray Q;
+    Q.ox = s_obj[0][wbase + o];
+    Q.oy = s_obj[1][wbase + o];
+    Q.oz = s_obj[2][wbase + o];
+    Q.Sx = s_obj[3][wbase + o];
+    Q.Sy = s_obj[4][wbase + o];
+    Q.Sz = s_obj[5][wbase + o];
+    Q.tmax = s_obj[6][wbase + o];
+    Q.tmin = tmin;
+    const int k = s_objk[wbase + o];
+    Q.kx = k & 3;
+    Q.ky = (k >> 2) & 3;
+    Q.kz = k >> 4;
+    const float4 a = __ldg(A.leaf + 3 * (size_t)slot), b = __ldg(A.leaf + 3 * (size_t)slot + 1),
+                 c = __ldg(A.leaf + 3 * (size_t)slot + 2);
+    const float v0[3] = {a.x, a.y, a.z}, v1[3] = {b.x, b.y, b.z}, v2[3] = {c.x, c.y, c.z};
+    id = __float_as_uint(a.w);
+    return isect_tri(Q, v0, v1, v2, t);
+  };
+  // folds a hit of instance ci into the ray's best (smallest t, then lowest
+  // instance, then lowest primitive)
+  auto take_hit = [&](float t, uint32_t id, uint32_t slot) {
+    const uint32_t bi = s_best[0][tid];
+    if (bi == kMiss || t < bt ||
+        (t == bt && (ci < bi || (ci == bi && id < __float_as_uint(__ldg(A.leaf + 3 * (size_t)s_best[1][tid]).w))))) {
+      s_best[0][tid] = ci;
+      s_best[1][tid] = slot;
       bt = t;
     }
   };
-  auto pop_top = [&]() {
-    while (tsp > 0) {
-      --tsp;
-      if (ttn[tsp] <= bt) {
-        cur = tref[tsp];
-        return;
+  // every queued test by all lanes (warp-uniform call)
+  auto flush = [&]() {
+    __syncwarp();
+    for (int b = 0; b < nq; b += 32) {
+      const int e = b + lane;
+      const bool on = e < nq;
+      const uint32_t slot = on ? qslot[e] : 0u;
+      const int o = on ? qlane[e] : lane;
+      const float tmin = __shfl_sync(FULL_MASK, P.tmin, o);
+      unsigned long long key = ~0ull;
+      uint32_t id;
+      float t;
+      if (on && tri_test(slot, o, tmin, id, t)) {
+        key = ((unsigned long long)t_order(t) << 32) | id;
+        atomicMin(&s_key[w][o], key);
       }
+      __syncwarp();
+      if (key != ~0ull && s_key[w][o] == key) s_kslot[w][o] = slot;  // one winner per owner
+      __syncwarp();
     }
-    done = true;
+    if (pending) {
+      const unsigned long long key = s_key[w][lane];
+      if (key != ~0ull) {
+        take_hit(t_from_order((uint32_t)(key >> 32)), (uint32_t)key, s_kslot[w][lane]);
+        s_key[w][lane] = ~0ull;
+      }
+      pending = false;
+    }
+    nq = 0;
+    __syncwarp();
   };
+  auto queue = [&](bool leaf, uint32_t slot) {
+    const unsigned m = __ballot_sync(FULL_MASK, leaf);
+    if (leaf) {
+      const int k = nq + __popc(m & lt);
+      qslot[k] = slot;
+      qlane[k] = (uint8_t)lane;
+      pending = true;
+    }
+    nq += __popc(m);
+  };
+
   while (true) {
     // Lanes whose rays finished take new ones once kInstRefill of the warp's
     // 32 are idle (rays differ widely in how many instances they enter).
@@ -179,30 +303,28 @@ __global__ void __launch_bounds__(kInstThreads) k_trace_inst(const Bvh2Node *tno
     const int n_idle = __popc(idle);
     if (!drained && (n_idle >= kInstRefill || n_idle == 32)) {
       unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(counter, (unsigned long long)n_idle);
+      if (lane == 0) base = atomicAdd(A.counter, (unsigned long long)n_idle);
       base = __shfl_sync(FULL_MASK, base, 0);
-      if (base + n_idle >= nrays) drained = true;
-      if (!active) {
-        const uint64_t mine = base + __popc(idle & lt);
-        if (mine < nrays) {
-          r = mine;
-          active = true;
-          done = false;
-          ray_setup(__ldg(rays + 2 * r), __ldg(rays + 2 * r + 1), W);
-          O = W;
-          best = kMiss;
-          binst = kMiss;
-          bslot = 0;
-          bt = W.tmax;
-          tsp = 0;
-          bsp = 0;
-          level = 0;
-          cur = 0;
-          if (ninst == 1) {
-            float tn;
-            cur = ~0;  // the single instance is the root leaf
-            if (!ray_box(W, troot[0], troot[1], troot[2], troot[3], troot[4], troot[5], bt, tn)) done = true;
-          }
+      if (base + n_idle >= A.nrays) drained = true;
+      const uint64_t r = base + __popc(idle & lt);
+      if (!active && r < A.nrays) {
+        Ray R;
+        ray_setup(__ldg(A.rays + 2 * r), __ldg(A.rays + 2 * r + 1), R);
+        active = true;
+        inside = false;
+        P = ray_pairs(R);
+        bt = R.tmax;
+        W.start();
+        s_obj[6][tid] = R.tmax;
+        s_best[0][tid] = kMiss;
+        s_key[w][lane] = ~0ull;
+        s_rid[tid] = r;
+        if (A.ninst == 1) {
+          float tn;
+          W.node = ~0;  // the single instance is the root leaf
+          W.t = R.tmin;
+          if (!ray_box(R, A.troot[0], A.troot[1], A.troot[2], A.troot[3], A.troot[4], A.troot[5], bt, tn))
+            W.node = kWalkEnd;
         }
       }
     }
@@ -210,125 +332,158 @@ __global__ void __launch_bounds__(kInstThreads) k_trace_inst(const Bvh2Node *tno
       if (drained) break;
       continue;
     }
-    if (active && !done) {
-      if (level == 1) {
-        // ---- bottom level: the instance's mesh in object space
-        const float4 *np = reinterpret_cast<const float4 *>(bvh + bnode);
-        const float4 f0 = __ldg(np), f1 = __ldg(np + 1), f2 = __ldg(np + 2);
-        const int4 rf = __ldg(reinterpret_cast<const int4 *>(np + 3));
-        float tn0, tn1;
-        bool h0 = ray_box(O, f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, bt, tn0) && tn0 <= bt;
-        bool h1 = ray_box(O, f1.z, f1.w, f2.x, f2.y, f2.z, f2.w, bt, tn1) && tn1 <= bt;
-        if (h0 && rf.x < 0) {
-          tri_test((uint32_t)~rf.x);
-          h0 = false;
+#pragma unroll 1
+    for (int step = 0; step < kInstSteps; ++step) {
+      const bool on = W.node >= 0;
+      float t0 = kNone, t1 = kNone;
+      int r0 = 0, r1 = 0;
+      bool leaf0 = false, leaf1 = false, found = false;
+      if (on && W.t <= bt) {
+        const Bvh2Node *nd = inside ? A.nodes + base_node + W.node : A.tnodes + W.node;
+        const ChildPairs c0 = load_child<V8>(&nd->c[0]), c1 = load_child<V8>(&nd->c[1]);
+        t0 = child_entry(c0, P, bt);
+        t1 = child_entry(c1, P, bt);
+        r0 = c0.ref;
+        r1 = c1.ref;
+        leaf0 = inside && r0 < 0 && t0 == t0;
+        leaf1 = inside && r1 < 0 && t1 == t1;
+        if (ANY) {
+          uint32_t id;
+          float t;
+          if (leaf0 && tri_test(base_leaf + (uint32_t)~r0, lane, P.tmin, id, t))
+            take_hit(t, id, base_leaf + (uint32_t)~r0);
+          if (leaf1 && t1 <= bt && tri_test(base_leaf + (uint32_t)~r1, lane, P.tmin, id, t))
+            take_hit(t, id, base_leaf + (uint32_t)~r1);
+          found = (leaf0 || leaf1) && s_best[0][tid] != kMiss;
         }
-        if (h1 && rf.y < 0) {
-          if (tn1 <= bt) tri_test((uint32_t)~rf.y);
-          h1 = false;
-        }
-        if (h1 && tn1 > bt) h1 = false;
-        if (ANY && best != kMiss) {
-          done = true;
-        } else if (h0 && h1) {
-          const bool first0 = tn0 <= tn1;
-          if (bsp < kInstStack) {
-            bstack[bsp++] = first0 ? rf.y : rf.x;
-            bnode = first0 ? rf.x : rf.y;
-          } else {
-            atomicCAS(err, 0u, 5u);  // traversal stack overflow
-            done = true;
-          }
-        } else if (h0) {
-          bnode = rf.x;
-        } else if (h1) {
-          bnode = rf.y;
-        } else if (bsp > 0) {
-          bnode = bstack[--bsp];
-        } else {
-          level = 0;  // back to the top level
-          pop_top();
-        }
-      } else if (cur >= 0) {
-        // ---- top level, inner node
-        const float4 *np = reinterpret_cast<const float4 *>(tnodes + cur);
-        const float4 f0 = __ldg(np), f1 = __ldg(np + 1), f2 = __ldg(np + 2);
-        const int4 rf = __ldg(reinterpret_cast<const int4 *>(np + 3));
-        float tn0, tn1;
-        const bool h0 = ray_box(W, f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, bt, tn0) && tn0 <= bt;
-        const bool h1 = ray_box(W, f1.z, f1.w, f2.x, f2.y, f2.z, f2.w, bt, tn1) && tn1 <= bt;
-        if (h0 && h1) {
-          const bool first0 = tn0 <= tn1;
-          if (tsp < kInstStack) {
-            tref[tsp] = first0 ? rf.y : rf.x;
-            ttn[tsp] = first0 ? tn1 : tn0;
-            ++tsp;
-            cur = first0 ? rf.x : rf.y;
-          } else {
-            atomicCAS(err, 0u, 5u);
-            done = true;
-          }
-        } else if (h0) {
-          cur = rf.x;
-        } else if (h1) {
-          cur = rf.y;
-        } else {
-          pop_top();
-        }
-      } else {
-        // ---- top level, an instance: enter its mesh in object space
-        ci = __ldg(tids + (uint32_t)~cur);
-        const uint32_t cm = __ldg(&inst[ci].custom_mask);
-        const uint32_t mesh = (uint32_t)__ldg(&inst[ci].blas);
-        bool entered = false;
-        if (((cm >> 24) & ray_mask) && mesh < im.meshes) {
-          const float *w = w2o + 12 * (size_t)ci;
-          if (__ldg(w) != 0.0f || __ldg(w + 1) != 0.0f || __ldg(w + 2) != 0.0f) {  // singular: all zero
-            ray_to_object(w, W, O);
-            const uint32_t b = im.tri_off ? __ldg(im.tri_off + mesh) : 0u;
-            const uint32_t cnt = im.tri_off ? __ldg(im.tri_off + mesh + 1) - b : im.n_all;
-            bvh = blas_all + (b - mesh);
-            leaf = leaf_all + 3 * (size_t)b;
-            if (cnt == 1) {
-              const float4 a = __ldg(leaf), bb = __ldg(leaf + 1), c = __ldg(leaf + 2);
-              float tn;
-              if (ray_box(O, fminf(a.x, fminf(bb.x, c.x)), fminf(a.y, fminf(bb.y, c.y)), fminf(a.z, fminf(bb.z, c.z)),
-                          fmaxf(a.x, fmaxf(bb.x, c.x)), fmaxf(a.y, fmaxf(bb.y, c.y)), fmaxf(a.z, fmaxf(bb.z, c.z)), bt,
+        if (leaf0) t0 = kNone;
+        if (leaf1) t1 = kNone;
+      }
+      if (!walk_next<kInstThreads, kInstShared, kInstDepth>(W, sh, over, on, t0, r0, t1, r1)) {
+        atomicCAS(A.err, 0u, 5u);  // traversal stack overflow
+        W.node = kWalkEnd;
+      }
+      if (ANY && found) W.node = kWalkEnd;
+      if (W.node == kWalkLeave) {  // back to the world ray; the next step pops
+        inside = false;
+        const unsigned long long r = s_rid[tid];
+        const float4 o = __ldg(A.rays + 2 * r), d = __ldg(A.rays + 2 * r + 1);
+        const float iz = __frcp_rn(d.z);
+        P.nxy = pk2(-o.x, -o.y);
+        P.nzz = pk2(-o.z, -o.z);
+        P.ixy = pk2(__frcp_rn(d.x), __frcp_rn(d.y));
+        P.izz = pk2(iz, iz);
+        W.node = 0;
+        W.t = kNone;
+      }
+      if (!ANY && __any_sync(FULL_MASK, leaf0 || leaf1)) {
+        if (nq > kInstQueue - 64) flush();
+        queue(leaf0, base_leaf + (uint32_t)~r0);
+        queue(leaf1, base_leaf + (uint32_t)~r1);
+      }
+    }
+    // ---- instances: enter them together
+    const unsigned walking = __ballot_sync(FULL_MASK, W.node >= 0);
+    const unsigned entering = __ballot_sync(FULL_MASK, W.node < 0 && W.node > kWalkLeave);
+    if (entering && (!walking || __popc(entering) >= kInstEnter)) {
+      const bool enter = W.node < 0 && W.node > kWalkLeave;
+      if (!ANY && __any_sync(FULL_MASK, enter && pending)) flush();
+      if (!ANY && nq > kInstQueue - 32) flush();
+      bool one = false, found = false;
+      if (enter) {
+        const uint32_t ti = __ldg(A.tids + (uint32_t)~W.node);
+        W.node = 0;  // the next step pops, unless the instance is entered below
+        const float t = W.t;
+        W.t = kNone;
+        const uint32_t cm = __ldg(&A.inst[ti].custom_mask);
+        const uint32_t mesh = (uint32_t)__ldg(&A.inst[ti].blas);
+        const float *wm = A.w2o + 12 * (size_t)ti;
+        if (t <= bt && ((cm >> 24) & A.ray_mask) && mesh < A.meshes &&
+            (__ldg(wm) != 0.0f || __ldg(wm + 1) != 0.0f || __ldg(wm + 2) != 0.0f)) {  // singular: all zero
+          const unsigned long long r = s_rid[tid];
+          const float4 o4 = __ldg(A.rays + 2 * r), d4 = __ldg(A.rays + 2 * r + 1);
+          Ray R, O;
+          R.ox = o4.x; R.oy = o4.y; R.oz = o4.z; R.tmin = o4.w;
+          R.dx = d4.x; R.dy = d4.y; R.dz = d4.z; R.tmax = d4.w;
+          ray_to_object(wm, R, O);
+          ci = ti;
+          base_leaf = A.tri_off ? __ldg(A.tri_off + mesh) : 0u;
+          const uint32_t cnt = A.tri_off ? __ldg(A.tri_off + mesh + 1) - base_leaf : A.n;
+          base_node = base_leaf - mesh;
+          s_obj[0][tid] = O.ox;
+          s_obj[1][tid] = O.oy;
+          s_obj[2][tid] = O.oz;
+          s_obj[3][tid] = O.Sx;
+          s_obj[4][tid] = O.Sy;
+          s_obj[5][tid] = O.Sz;
+          s_objk[tid] = O.kx | (O.ky << 2) | (O.kz << 4);
+          if (cnt == 1) {
+            const float4 a = __ldg(A.leaf + 3 * (size_t)base_leaf), b = __ldg(A.leaf + 3 * (size_t)base_leaf + 1),
+                         c = __ldg(A.leaf + 3 * (size_t)base_leaf + 2);
+            float tn;
+            one = ray_box(O, fminf(a.x, fminf(b.x, c.x)), fminf(a.y, fminf(b.y, c.y)), fminf(a.z, fminf(b.z, c.z)),
+                          fmaxf(a.x, fmaxf(b.x, c.x)), fmaxf(a.y, fmaxf(b.y, c.y)), fmaxf(a.z, fmaxf(b.z, c.z)), bt,
                           tn) &&
-                  tn <= bt)
-                tri_test(0);
-              if (ANY && best != kMiss) done = true;
-            } else {
-              level = 1;
-              bnode = 0;
-              bsp = 0;
-              entered = true;
+                  tn <= bt;
+            if (ANY && one) {
+              uint32_t id;
+              float th;
+              if (tri_test(base_leaf, lane, P.tmin, id, th)) {
+                take_hit(th, id, base_leaf);
+                found = true;
+              }
+            }
+          } else {
+            P = ray_pairs(O);
+            inside = true;
+            W.t = t;
+            if (!walk_push<kInstThreads, kInstShared, kInstDepth>(W, sh, over, kWalkLeave, 0.0f)) {
+              atomicCAS(A.err, 0u, 5u);
+              W.node = kWalkEnd;
             }
           }
         }
-        if (!entered && !done) pop_top();
+      }
+      if (ANY) {
+        if (found) W.node = kWalkEnd;
+      } else {
+        __syncwarp();
+        queue(one, base_leaf);
       }
     }
-    if (active && done) {
-      Hit h;
-      h.prim = best;
-      h.t = __int_as_float(0x7f800000);
-      if (best != kMiss) {
-        // the winner's object-space ray again (same operations, same bits)
-        ray_to_object(w2o + 12 * (size_t)binst, W, O);
-        const uint32_t mesh = (uint32_t)__ldg(&inst[binst].blas);
-        const uint32_t b = im.tri_off ? __ldg(im.tri_off + mesh) : 0u;
-        const float4 *lf = leaf_all + 3 * (size_t)b;
-        const float4 a = __ldg(lf + 3 * (size_t)bslot), bb = __ldg(lf + 3 * (size_t)bslot + 1),
-                     c = __ldg(lf + 3 * (size_t)bslot + 2);
-        const float v0[3] = {a.x, a.y, a.z}, v1[3] = {bb.x, bb.y, bb.z}, v2[3] = {c.x, c.y, c.z};
-        h.t = refine_t(O, v0, v1, v2);
+    const bool done = W.node == kWalkEnd;
+    if (!ANY) {
+      const unsigned waiting = __ballot_sync(FULL_MASK, done && active && pending);
+      const unsigned running = __ballot_sync(FULL_MASK, active && !done);
+      if (nq >= kInstFlush || (waiting && (!running || 32 - __popc(running) >= kInstRefill))) flush();
+    }
+    const bool fin = active && done && !pending;
+    if (__any_sync(FULL_MASK, fin)) {
+      const bool hit = fin && s_best[0][tid] != kMiss;
+      if (fin && !hit) {
+        const unsigned long long r = s_rid[tid];
+        Hit h;
+        h.prim = kMiss;
+        h.t = __int_as_float(0x7f800000);
+        A.hits[r] = h;
+        if (A.hit_inst) A.hit_inst[r] = kMiss;
       }
-      hits[r] = h;
-      if (hit_inst) hit_inst[r] = binst;
-      active = false;
+      const unsigned m = __ballot_sync(FULL_MASK, hit);
+      if (hit) {
+        const int k = nrq + __popc(m & lt);
+        rq.ray[k] = s_rid[tid];
+        rq.inst[k] = s_best[0][tid];
+        rq.slot[k] = s_best[1][tid];
+      }
+      nrq += __popc(m);
+      if (nrq >= 32) {
+        nrq -= 32;
+        inst_refine(A, rq, nrq, 32);
+      }
+      if (fin) active = false;
     }
   }
+  inst_refine(A, rq, 0, nrq);
 }
 
 }  // namespace gprtcu
@@ -371,18 +526,32 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuTraceInstances(const gprtcuLbvh *tlas, 
   ScratchHeader *hdr = (ScratchHeader *)scratch;
   unsigned long long *counter = reinterpret_cast<unsigned long long *>(&hdr->ticket[0]);
   GPRTCU_TRY(cudaMemsetAsync(scratch, 0, sizeof(ScratchHeader), stream));
-  const int blocks = gprtcu_num_sms() * 8;
+  const int blocks = gprtcu_num_sms() * kInstCtas;
   const uint64_t need = (numRays + kInstThreads - 1) / kInstThreads;
   const int grid = (int)(need < (uint64_t)blocks ? need : blocks);
-  const InstMeshes im{numMeshes > 1 ? triOffsets : nullptr, numMeshes, blas->numPrims};
-#define GPRTCU_ITRACE(A)                                                                                             \
-  k_trace_inst<A><<<grid, kInstThreads, 0, stream>>>(                                                              \
-      (const Bvh2Node *)tlas->bvh2, tlas->ids, tlas->numPrims, tlas->rootBox, (const InstanceRec *)instances,     \
-      worldToObject, (const Bvh2Node *)blas->bvh2, (const float4 *)blas->leafTris, im, (const float4 *)rays, numRays, \
-      rayMask, (Hit *)hits, hitInstance, counter, &hdr->status)
-  if (anyHit) GPRTCU_ITRACE(true);
-  else GPRTCU_ITRACE(false);
-#undef GPRTCU_ITRACE
+  InstArgs a;
+  a.tnodes = (const Bvh2Node *)tlas->bvh2;
+  a.tids = tlas->ids;
+  a.ninst = tlas->numPrims;
+  a.troot = tlas->rootBox;
+  a.inst = (const InstanceRec *)instances;
+  a.w2o = worldToObject;
+  a.nodes = (const Bvh2Node *)blas->bvh2;
+  a.leaf = (const float4 *)blas->leafTris;
+  a.tri_off = numMeshes > 1 ? triOffsets : nullptr;
+  a.meshes = numMeshes;
+  a.n = blas->numPrims;
+  a.rays = (const float4 *)rays;
+  a.nrays = numRays;
+  a.ray_mask = rayMask;
+  a.hits = (Hit *)hits;
+  a.hit_inst = hitInstance;
+  a.counter = counter;
+  a.err = &hdr->status;
+  auto launch = [&](auto kernel) { kernel<<<grid, kInstThreads, 0, stream>>>(a); };
+  const bool v8 = (((uintptr_t)tlas->bvh2 | (uintptr_t)blas->bvh2) & 31) == 0;
+  if (anyHit) v8 ? launch(k_trace_inst<true, true>) : launch(k_trace_inst<true, false>);
+  else v8 ? launch(k_trace_inst<false, true>) : launch(k_trace_inst<false, false>);
   GPRTCU_TRY(cudaGetLastError());
   return GPRTCU_OK;
 }

@@ -408,9 +408,9 @@ __global__ void __launch_bounds__(256, 8) k_karras(const uint32_t *codes, const 
       // arrival waits to see replaced (no float box bound has this pattern)
       int4 *q = reinterpret_cast<int4 *>(&bvh[inner_base + i]);
       q[0] = make_int4(-1, -1, -1, -1);
-      q[1] = make_int4(-1, -1, -1, -1);
+      q[1] = make_int4(-1, -1, lleaf ? ~(int)left : (int)lc, 0);
       q[2] = make_int4(-1, -1, -1, -1);
-      q[3] = make_int4(lleaf ? ~(int)left : (int)lc, rleaf ? ~(int)right : (int)rc, 0, 0);
+      q[3] = make_int4(-1, -1, rleaf ? ~(int)right : (int)rc, 0);
     }
   }
 }
@@ -429,17 +429,37 @@ __global__ void __launch_bounds__(256, 8) k_karras(const uint32_t *codes, const 
 // triangles: build 17.6 -> 15.5 ms without it).  Without traversal nodes the
 // sibling's box is read from the reference-layout array after an
 // acquire-release count.
+// A16: traversal nodes on 16-byte boundaries (a build requires them; a refit
+// alone also takes 8-byte ones).
+template <bool A16> __device__ __forceinline__ void refit_store_box(float *o, const float *b) {
+  if constexpr (A16) {
+    *reinterpret_cast<float4 *>(o) = make_float4(b[0], b[1], b[3], b[4]);
+    *reinterpret_cast<float2 *>(o + 4) = make_float2(b[2], b[5]);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) o[box_word(k)] = b[k];
+  }
+}
 // The sibling's box from its slot of the parent's traversal node (L2, not
 // L1); false while a word still holds the all-ones "not formed" pattern.
-__device__ __forceinline__ bool refit_read_box(const float2 *o2, float *sb) {
+template <bool A16> __device__ __forceinline__ bool refit_read_box(const float *o, float *sb) {
+  float w[6];
+  if constexpr (A16) {
+    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3])
+                 : "l"(o)
+                 : "memory");
+    asm volatile("ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];" : "=f"(w[4]), "=f"(w[5]) : "l"(o + 4) : "memory");
+  } else {
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(w[k]) : "l"(o + k) : "memory");
+  }
   bool ready = true;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float2 t;
-    asm volatile("ld.relaxed.gpu.global.v2.f32 {%0, %1}, [%2];" : "=f"(t.x), "=f"(t.y) : "l"(o2 + k) : "memory");
-    sb[2 * k] = t.x;
-    sb[2 * k + 1] = t.y;
-    ready &= __float_as_uint(t.x) != 0xFFFFFFFFu && __float_as_uint(t.y) != 0xFFFFFFFFu;
+  for (int k = 0; k < 6; ++k) {
+    ready &= __float_as_uint(w[k]) != 0xFFFFFFFFu;
+    sb[k] = w[box_word(k)];
   }
   return ready;
 }
@@ -449,7 +469,7 @@ __device__ __forceinline__ bool refit_read_box(const float2 *o2, float *sb) {
 __constant__ int64_t c_refit_skip = -1;
 __constant__ uint32_t c_refit_budget = DEFAULT_SPIN_BUDGET;
 
-template <int KIND, bool BATCHED>
+template <int KIND, bool BATCHED, bool A16>
 __global__ void __launch_bounds__(256, 8) k_refit(const float *pos, const uint32_t *tri, const uint32_t *ids,
                                                const uint64_t *keys, MeshMap mm, int4 *nodes, float *aabbs,
                                                Bvh2Node *bvh, float4 *leaf_tris, uint32_t *codes_out,
@@ -514,10 +534,7 @@ __global__ void __launch_bounds__(256, 8) k_refit(const float *pos, const uint32
     // (a hooked leaf, at its first step, leaves its slot unwritten)
     const bool skip_store = hooked && child == leaf;
     if (bvh && !skip_store) {
-      float2 *cb = reinterpret_cast<float2 *>(bvh[inner_base + p].box + 6 * side);
-      cb[0] = make_float2(bx[0], bx[1]);
-      cb[1] = make_float2(bx[2], bx[3]);
-      cb[2] = make_float2(bx[4], bx[5]);
+      refit_store_box<A16>(bvh[inner_base + p].c[side].box, bx);
     }
     // first arrival: the sibling finishes
     if (bvh) {
@@ -534,12 +551,12 @@ __global__ void __launch_bounds__(256, 8) k_refit(const float *pos, const uint32
     // the next parent's node, loaded while the sibling's box is read
     int4 gpn = make_int4(0, 0, -1, -1);
     if (pn.z >= 0) gpn = nodes[node_base + pn.z];
-    const float *ob = bvh ? bvh[inner_base + p].box + 6 * rd : aabbs + 6 * (size_t)(node_base + sib);
+    const float *ob = bvh ? bvh[inner_base + p].c[rd].box : aabbs + 6 * (size_t)(node_base + sib);
     float sb[6];
     if (bvh) {
       // bounded wait for the sibling's stores; a wait that runs out records
       // GPRTCU_ERR_TIMEOUT in the scratch header
-      for (uint32_t spin = 0; !refit_read_box(reinterpret_cast<const float2 *>(ob), sb); ++spin)
+      for (uint32_t spin = 0; !refit_read_box<A16>(ob, sb); ++spin)
         if (spin == c_refit_budget) {
           record_error(lbvh_header(), GPRTCU_ERR_TIMEOUT);
           break;
@@ -621,7 +638,7 @@ void launch_build(const float *pos, const uint32_t *tri, MeshMap mm, int codeKin
                                                                                          sort_status);
     // traversal nodes for triangles and user-primitive boxes; leaf-order
     // triangles for triangles only
-    k_refit<KIND, BATCHED><<<(unsigned)((mm.n + 255) / 256), 256, 0, stream>>>(
+    k_refit<KIND, BATCHED, true><<<(unsigned)((mm.n + 255) / 256), 256, 0, stream>>>(
         pos, tri, out->ids, keys, mm, nodes, out->aabbs, (KIND == 0 || KIND == 3) ? (Bvh2Node *)out->bvh2 : nullptr,
         KIND == 0 ? (float4 *)out->leafTris : nullptr, out->codes, arrivals, out->rootBox, sort_status);
   }
@@ -725,16 +742,16 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuLbvhRefitTriangles(const float *positio
   const MeshMap mm{numMeshes > 1 ? triOffsets : nullptr, numMeshes, n};
   // the traversal nodes' child boxes back to all-ones (the refit waits for them to change)
   if (bvh->bvh2 && n > numMeshes)
-    GPRTCU_TRY(cudaMemset2DAsync(bvh->bvh2, sizeof(Bvh2Node), 0xFF, 12 * sizeof(float), n - numMeshes, stream));
+    GPRTCU_TRY(cudaMemset2DAsync(bvh->bvh2, sizeof(Bvh2Child), 0xFF, 6 * sizeof(float), 2 * (size_t)(n - numMeshes), stream));
   const unsigned grid = (unsigned)((n + 255) / 256);
-  if (numMeshes > 1)
-    k_refit<0, true><<<grid, 256, 0, stream>>>(positions, triangles, bvh->ids, nullptr, mm, (int4 *)bvh->nodes,
-                                               bvh->aabbs, (Bvh2Node *)bvh->bvh2, (float4 *)bvh->leafTris, nullptr,
-                                               arrivals, bvh->rootBox, nullptr);
-  else
-    k_refit<0, false><<<grid, 256, 0, stream>>>(positions, triangles, bvh->ids, nullptr, mm, (int4 *)bvh->nodes,
-                                                bvh->aabbs, (Bvh2Node *)bvh->bvh2, (float4 *)bvh->leafTris, nullptr,
-                                                arrivals, bvh->rootBox, nullptr);
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, 256, 0, stream>>>(positions, triangles, bvh->ids, nullptr, mm, (int4 *)bvh->nodes, bvh->aabbs,
+                                     (Bvh2Node *)bvh->bvh2, (float4 *)bvh->leafTris, nullptr, arrivals, bvh->rootBox,
+                                     nullptr);
+  };
+  const bool a16 = ((uintptr_t)bvh->bvh2 & 15) == 0;
+  if (numMeshes > 1) a16 ? launch(k_refit<0, true, true>) : launch(k_refit<0, true, false>);
+  else a16 ? launch(k_refit<0, false, true>) : launch(k_refit<0, false, false>);
   GPRTCU_TRY(cudaGetLastError());
   return GPRTCU_OK;
 }

@@ -316,10 +316,10 @@ __global__ void __launch_bounds__(kLocateThreads) k_locate_solids(const Bvh2Node
       uint32_t c0 = kNoCell, c1 = kNoCell;  // leaf candidates of this step
       if (!done) {
         const float4 *np = reinterpret_cast<const float4 *>(bvh + node);
-        const float4 f0 = __ldg(np), f1 = __ldg(np + 1), f2 = __ldg(np + 2);
-        const int4 rf = __ldg(reinterpret_cast<const int4 *>(np + 3));
-        bool h0 = point_in(p.x, p.y, p.z, f0.x, f0.y, f0.z, f0.w, f1.x, f1.y);
-        bool h1 = point_in(p.x, p.y, p.z, f1.z, f1.w, f2.x, f2.y, f2.z, f2.w);
+        const float4 g0 = __ldg(np), g1 = __ldg(np + 1), g2 = __ldg(np + 2), g3 = __ldg(np + 3);
+        const int2 rf = make_int2(__float_as_int(g1.z), __float_as_int(g3.z));
+        bool h0 = point_in(p.x, p.y, p.z, g0.x, g0.y, g1.x, g0.z, g0.w, g1.y);
+        bool h1 = point_in(p.x, p.y, p.z, g2.x, g2.y, g3.x, g2.z, g2.w, g3.y);
         if (h0 && rf.x < 0) {
           c0 = __ldg(ids + (uint32_t)~rf.x);
           h0 = false;

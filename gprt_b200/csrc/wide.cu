@@ -55,8 +55,9 @@ enum { C_LO = 0, C_HI = 1, C_TAIL = 2, C_LEAF = 3, C_TICKET = 4 };
 // depth stay below 62.
 constexpr int kWideMaxLevels = 62;
 
+// (a box in the order of Bvh2Child::box)
 __device__ __forceinline__ float box_area(const float *b) {
-  const float dx = b[3] - b[0], dy = b[4] - b[1], dz = b[5] - b[2];
+  const float dx = b[2] - b[0], dy = b[3] - b[1], dz = b[5] - b[4];
   return dx * dy + dy * dz + dz * dx;
 }
 
@@ -152,10 +153,10 @@ __global__ void __launch_bounds__(128) k_wide_level(const Bvh2Node *bvh2, const 
         const Bvh2Node nd = mb[it.bref];
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          ref[c] = nd.ref[c];
+          ref[c] = nd.c[c].ref;
 #pragma unroll
-          for (int k = 0; k < 6; ++k) CBOX(c, k) = nd.box[6 * c + k];
-          area[c] = box_area(nd.box + 6 * c);
+          for (int k = 0; k < 6; ++k) CBOX(c, k) = nd.c[c].box[box_word(k)];
+          area[c] = box_area(nd.c[c].box);
         }
         cnt = 2;
         // greedy: replace the inner child of largest area (lowest slot on
@@ -175,20 +176,20 @@ __global__ void __launch_bounds__(128) k_wide_level(const Bvh2Node *bvh2, const 
           for (int c = 0; c < 8; ++c)
             if (c == best) rb = ref[c];
           const Bvh2Node ch = mb[rb];
-          const float a0 = box_area(ch.box), a1 = box_area(ch.box + 6);
+          const float a0 = box_area(ch.c[0].box), a1 = box_area(ch.c[1].box);
 #pragma unroll
           for (int k = 0; k < 6; ++k) {
-            CBOX(best, k) = ch.box[k];
-            CBOX(cnt, k) = ch.box[6 + k];
+            CBOX(best, k) = ch.c[0].box[box_word(k)];
+            CBOX(cnt, k) = ch.c[1].box[box_word(k)];
           }
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             if (c == best) {
-              ref[c] = ch.ref[0];
+              ref[c] = ch.c[0].ref;
               area[c] = a0;
             }
             if (c == cnt) {
-              ref[c] = ch.ref[1];
+              ref[c] = ch.c[1].ref;
               area[c] = a1;
             }
           }
@@ -304,47 +305,6 @@ __device__ __forceinline__ float scale_of(int8_t e) { return __int_as_float(((in
 // 2^15 x the node's quantisation step (infinity past the float range: the
 // axis then gives NaN and drops out of the box test, which stays conservative)
 __device__ __forceinline__ float scale15_of(int8_t e) { return __int_as_float(min((int)e + 142, 255) << 23); }
-
-// Packed pairs of fp32 (sm_100 f32x2 arithmetic; each half rounds as the
-// scalar instruction would) and three-input min / max.
-__device__ __forceinline__ unsigned long long pk2(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void up2(unsigned long long v, float &a, float &b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long fma2_rd(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ unsigned long long fma2_ru(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rp.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ unsigned long long add2_rn(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long mul2_rn(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-__device__ __forceinline__ float min3f(float a, float b, float c) {
-  float r;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
 
 __device__ __forceinline__ void wide_leaf_test(const float4 *leaf, uint32_t i, const Ray &R, uint32_t &best,
                                                uint32_t &best_leaf, float &bt) {
@@ -676,17 +636,6 @@ __global__ void __launch_bounds__(kWideThreads, 8)
       active = false;
     }
   }
-}
-
-// Order-preserving unsigned image of a distance with -0 and +0 merged:
-// comparing (t_order(t) << 32 | id) as 64-bit unsigned integers compares
-// (t, id) as the immediate test does (smaller t first, then the lower id).
-__device__ __forceinline__ uint32_t t_order(float t) {
-  const uint32_t u = t == 0.0f ? 0u : __float_as_uint(t);
-  return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
-}
-__device__ __forceinline__ float t_from_order(uint32_t k) {
-  return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k);
 }
 
 constexpr int kLeafFlush = 24;  // queued triangle tests that trigger a flush

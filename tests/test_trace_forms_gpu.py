@@ -1,0 +1,120 @@
+"""Binary traversal over the forms its launch rule tells apart: few rays (spread
+over the warps, fewer than 32 to a warp) up to full warps with a ragged end,
+traversal nodes on 32-byte boundaries or only on 16-byte ones, one mesh or a
+batch with one-triangle meshes; and a refit into nodes that are only 8-byte
+aligned.  Ids and t bits equal the oracle's traversal of the same tree."""
+import numpy as np
+import pytest
+
+import oracle
+from gprt_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _shift_nodes(bvh, nbytes):
+    """Moves the traversal nodes to `nbytes` past a 256-byte boundary."""
+    import torch
+    words = bvh.bvh2.numel()
+    buf = torch.zeros(words + 64, dtype=torch.float32, device="cuda")
+    assert buf.data_ptr() % 256 == 0
+    k = nbytes // 4
+    bvh.bvh2 = buf[k:k + words].view(-1, 16)
+    bvh.desc.bvh2 = bvh.bvh2.data_ptr()
+
+
+def _expect(pos, tri, rays):
+    return oracle.trace_lbvh(pos, tri, oracle.lbvh_build_tri(pos, tri), rays)
+
+
+def _same(got, exp):
+    hit = exp["prim"] != 0xFFFFFFFF
+    return np.array_equal(got["prim"], exp["prim"]) and np.array_equal(got["t"][hit].view(np.uint32),
+                                                                       exp["t"][hit].view(np.uint32))
+
+
+@pytest.mark.parametrize("shift", [0, 16, 32])
+@pytest.mark.parametrize("n,m", [(1, 3), (2, 1), (3, 33), (700, 4099), (5000, 18943), (5000, 18945), (20000, 200003)])
+def test_trace_forms(cuda, n, m, shift):
+    import torch
+    from gprt_b200 import api
+    pos, tri = scenes.soup(n, seed=n + m, sigma=0.02 if n > 100 else 0.3)
+    rays = scenes.rays(m, seed=m)
+    p, t, r = torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda(), torch.from_numpy(rays).cuda()
+    b = api.Lbvh(n)
+    _shift_nodes(b, shift)
+    api.lbvh_build_triangles(p, t, b)
+    exp = _expect(pos, tri, rays)
+    assert _same(api.hits_numpy(api.trace(b, r)), exp)
+    anyh = api.hits_numpy(api.trace(b, r, anyhit=True))
+    assert np.array_equal(anyh["prim"] != 0xFFFFFFFF, exp["prim"] != 0xFFFFFFFF)
+
+
+@pytest.mark.parametrize("shift", [0, 16])
+def test_batch_trace_forms(cuda, shift):
+    import torch
+    from gprt_b200 import api
+    sizes = [1, 700, 1, 1, 33, 2, 4000]
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    pos, tri = scenes.soup(int(off[-1]), seed=4, sigma=0.05)
+    rays = scenes.rays(int(off[-1]) * 3, seed=5)
+    roff = off * 3
+    b = api.BatchLbvh(off)
+    _shift_nodes(b, shift)
+    api.batch_build_triangles(torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda(), b)
+    ro = torch.from_numpy(roff.astype(np.int32)).cuda()
+    got = api.hits_numpy(api.batch_trace(b, torch.from_numpy(rays).cuda(), ro))
+    for k in range(len(sizes)):
+        t = np.ascontiguousarray(tri[off[k]:off[k + 1]])
+        assert _same(got[roff[k]:roff[k + 1]], _expect(pos, t, rays[roff[k]:roff[k + 1]])), k
+
+
+@pytest.mark.parametrize("shift", [0, 8, 16])
+def test_refit_node_alignment(cuda, shift):
+    """A refit writes the same traversal nodes wherever they lie."""
+    import torch
+    from gprt_b200 import api
+    n = 3001
+    pos, tri = scenes.soup(n, seed=8, sigma=0.05)
+    p, t = torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda()
+    b = api.lbvh_build_triangles(p, t)
+    want = api.lbvh_refit_triangles(p * 0.5 + 0.1, t, b).bvh2.clone()
+    api.lbvh_refit_triangles(p, t, b)
+    keep = b.bvh2.clone()
+    _shift_nodes(b, shift)
+    b.bvh2.copy_(keep)
+    api.lbvh_refit_triangles(p * 0.5 + 0.1, t, b)
+    assert torch.equal(b.bvh2.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("anyhit", [False, True])
+def test_instance_node_alignment(cuda, anyhit):
+    """Instanced traversal gives the same hits wherever the nodes of the two
+    levels lie (mesh sizes include one triangle, a deep mix of levels)."""
+    import torch
+    from gprt_b200 import api
+    rng = np.random.default_rng(3)
+    sizes = [1, 900, 40, 1, 5000]
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    pos, tri = scenes.soup(int(off[-1]), seed=6, sigma=0.05)
+    p, t = torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda()
+    n = 300
+    rec = np.zeros(n, np.dtype(api.INSTANCE_DTYPE))
+    q, _ = np.linalg.qr(rng.normal(size=(n, 3, 3)))
+    m = np.concatenate([q * rng.uniform(0.5, 1.5, (n, 1, 1)), rng.uniform(0, 4, (n, 3, 1))], 2)
+    rec["transform"] = m.reshape(n, 12)
+    rec["custom_mask"] = 0xFF << 24
+    rec["blas"] = np.arange(n) % len(sizes)
+    rays = torch.from_numpy(scenes.rays(20011, seed=9) * np.array([4, 4, 4, 1, 1, 1, 1, 1], np.float32)).cuda()
+    out = []
+    for shift in (0, 16):
+        b = api.BatchLbvh(off)
+        _shift_nodes(b, shift)
+        api.batch_build_triangles(p, t, b)
+        tlas = api.Tlas(api.instances_tensor(rec), b.root, len(sizes))
+        _shift_nodes(tlas.bvh, shift)
+        tlas.build()
+        h, i = api.trace_instances(tlas, b, rays, b.tri_off, len(sizes), anyhit=anyhit)
+        out.append((h.clone(), i.clone()))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert int((out[0][1] >= 0).sum()) > 100
