@@ -124,6 +124,7 @@ struct InstArgs {
   const float4 *rays;
   uint64_t nrays;
   uint32_t ray_mask;
+  int lanes;  // rays a warp holds at a time
   Hit *hits;
   uint32_t *hit_inst;
   unsigned long long *counter;
@@ -297,17 +298,9 @@ __global__ void __launch_bounds__(kInstThreads, kInstCtas) k_trace_inst(const In
   };
 
   while (true) {
-    // Lanes whose rays finished take new ones once kInstRefill of the warp's
-    // 32 are idle (rays differ widely in how many instances they enter).
-    const unsigned idle = __ballot_sync(FULL_MASK, !active);
-    const int n_idle = __popc(idle);
-    if (!drained && (n_idle >= kInstRefill || n_idle == 32)) {
-      unsigned long long base = 0;
-      if (lane == 0) base = atomicAdd(A.counter, (unsigned long long)n_idle);
-      base = __shfl_sync(FULL_MASK, base, 0);
-      if (base + n_idle >= A.nrays) drained = true;
-      const uint64_t r = base + __popc(idle & lt);
-      if (!active && r < A.nrays) {
+    {
+      uint64_t r;
+      if (warp_take(active, drained, A.lanes, kInstRefill, A.nrays, A.counter, r)) {
         Ray R;
         ray_setup(__ldg(A.rays + 2 * r), __ldg(A.rays + 2 * r + 1), R);
         active = true;
@@ -455,7 +448,7 @@ __global__ void __launch_bounds__(kInstThreads, kInstCtas) k_trace_inst(const In
     if (!ANY) {
       const unsigned waiting = __ballot_sync(FULL_MASK, done && active && pending);
       const unsigned running = __ballot_sync(FULL_MASK, active && !done);
-      if (nq >= kInstFlush || (waiting && (!running || 32 - __popc(running) >= kInstRefill))) flush();
+      if (nq >= kInstFlush || (waiting && (!running || A.lanes - __popc(running) >= kInstRefill))) flush();
     }
     const bool fin = active && done && !pending;
     if (__any_sync(FULL_MASK, fin)) {
@@ -526,9 +519,7 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuTraceInstances(const gprtcuLbvh *tlas, 
   ScratchHeader *hdr = (ScratchHeader *)scratch;
   unsigned long long *counter = reinterpret_cast<unsigned long long *>(&hdr->ticket[0]);
   GPRTCU_TRY(cudaMemsetAsync(scratch, 0, sizeof(ScratchHeader), stream));
-  const int blocks = gprtcu_num_sms() * kInstCtas;
-  const uint64_t need = (numRays + kInstThreads - 1) / kInstThreads;
-  const int grid = (int)(need < (uint64_t)blocks ? need : blocks);
+  const RayGrid g = ray_grid(numRays, kInstCtas, kInstWarps);
   InstArgs a;
   a.tnodes = (const Bvh2Node *)tlas->bvh2;
   a.tids = tlas->ids;
@@ -544,11 +535,12 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuTraceInstances(const gprtcuLbvh *tlas, 
   a.rays = (const float4 *)rays;
   a.nrays = numRays;
   a.ray_mask = rayMask;
+  a.lanes = g.lanes;
   a.hits = (Hit *)hits;
   a.hit_inst = hitInstance;
   a.counter = counter;
   a.err = &hdr->status;
-  auto launch = [&](auto kernel) { kernel<<<grid, kInstThreads, 0, stream>>>(a); };
+  auto launch = [&](auto kernel) { kernel<<<g.ctas, kInstThreads, 0, stream>>>(a); };
   const bool v8 = (((uintptr_t)tlas->bvh2 | (uintptr_t)blas->bvh2) & 31) == 0;
   if (anyHit) v8 ? launch(k_trace_inst<true, true>) : launch(k_trace_inst<true, false>);
   else v8 ? launch(k_trace_inst<false, true>) : launch(k_trace_inst<false, false>);

@@ -16,6 +16,7 @@ namespace gprtcu {
 
 constexpr int kTraceThreads = 128;
 constexpr int kTraceWarps = kTraceThreads / 32;
+constexpr int kTraceCtas = 8;     // per SM: 64 registers
 constexpr int kStackShared = 8;  // stack entries in shared memory
 constexpr int kStackDepth = 64;
 
@@ -117,26 +118,15 @@ __device__ __forceinline__ void finish_rays(const TraceArgs &A, RefineQueue &q, 
   }
 }
 
-// Idle lanes take new rays once kTraceRefill of the warp's A.lanes are idle
-// (or all are).  Returns true on the lanes that took one; base_leaf and
-// base_node are the first leaf slot and node of the ray's mesh and n its
-// triangles.
+// Idle lanes take new rays (warp_take).  Returns true on the lanes that took
+// one; base_leaf and base_node are the first leaf slot and node of the ray's
+// mesh and n its triangles.
 constexpr int kTraceRefill = 8;
 
 template <bool BATCHED>
 __device__ __forceinline__ bool take_rays(const TraceArgs &A, bool active, bool &drained, uint64_t &r, Ray &R,
                                           uint32_t &n, uint32_t &base_leaf, uint32_t &base_node) {
-  const int lane = threadIdx.x & 31;
-  const unsigned idle = __ballot_sync(FULL_MASK, !active && lane < A.lanes);
-  const int n_idle = __popc(idle);
-  if (drained || (n_idle < kTraceRefill && n_idle < A.lanes)) return false;
-  unsigned long long base = 0;
-  if (lane == 0) base = atomicAdd(A.counter, (unsigned long long)n_idle);
-  base = __shfl_sync(FULL_MASK, base, 0);
-  if (base + n_idle >= A.nrays) drained = true;
-  const uint64_t mine = base + __popc(idle & ((1u << lane) - 1u));
-  if (active || lane >= A.lanes || mine >= A.nrays) return false;
-  r = mine;
+  if (!warp_take(active, drained, A.lanes, kTraceRefill, A.nrays, A.counter, r)) return false;
   ray_setup(__ldg(A.rays + 2 * r), __ldg(A.rays + 2 * r + 1), R);
   n = A.n;
   base_leaf = base_node = 0;
@@ -153,7 +143,7 @@ __device__ __forceinline__ bool take_rays(const TraceArgs &A, bool active, bool 
 // Any hit: a lane tests the leaf triangles it meets at once, and the first
 // step with a hit ends its ray.
 template <bool BATCHED, bool V8>
-__global__ void __launch_bounds__(kTraceThreads, 8) k_trace_any(const TraceArgs A) {
+__global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_any(const TraceArgs A) {
   __shared__ float2 s_stack[kStackShared][kTraceThreads];
   __shared__ RefineQueue s_rq[kTraceWarps];
   RefineQueue &rq = s_rq[threadIdx.x >> 5];
@@ -243,7 +233,7 @@ constexpr int kSteps = 6;  // node steps between two looks at what else is to be
 constexpr int kLeafQueue = 96;  // a step queues at most 64
 
 template <bool BATCHED, bool V8>
-__global__ void __launch_bounds__(kTraceThreads, 8) k_trace_closest(const TraceArgs A) {
+__global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_closest(const TraceArgs A) {
   __shared__ float2 s_stack[kStackShared][kTraceThreads];
   __shared__ RefineQueue s_rq[kTraceWarps];
   __shared__ uint32_t s_qslot[kTraceWarps][kLeafQueue];
@@ -423,18 +413,7 @@ gprtcuStatus trace_launch(const gprtcuLbvh *bvh, const uint32_t *tri_off, const 
   ScratchHeader *hdr = (ScratchHeader *)scratch;
   unsigned long long *counter = reinterpret_cast<unsigned long long *>(&hdr->ticket[0]);
   GPRTCU_TRY(cudaMemsetAsync(scratch, 0, sizeof(ScratchHeader), stream));
-  const int blocks = gprtcu_num_sms() * 8;  // 64 registers: 8 CTAs of 128 threads per SM
-  // Rays per warp: all 32 lanes once there are rays for every warp that fits
-  // on the GPU; with fewer rays they are spread over the warps instead, at
-  // least four to each (a warp's time is that of its longest ray, and lanes
-  // without a ray still run queued triangle tests).  4,099 rays on 1,501
-  // triangles at 32 / 16 / 8 / 4 / 2 / 1 rays per warp: 102 / 85 / 81 / 78 /
-  // 78 / 93 us.
-  const uint64_t warps = (uint64_t)blocks * kTraceWarps;
-  const uint64_t share = (nrays + warps - 1) / warps;
-  const int lanes = share >= 32 ? 32 : (share < 4 ? 4 : (int)share);
-  const uint64_t need = (nrays + lanes * kTraceWarps - 1) / (lanes * kTraceWarps);
-  const int grid = (int)(need < (uint64_t)blocks ? need : blocks);
+  const RayGrid g = ray_grid(nrays, kTraceCtas, kTraceWarps);
   TraceArgs a;
   a.bvh = (const Bvh2Node *)bvh->bvh2;
   a.leaf = (const float4 *)bvh->leafTris;
@@ -442,7 +421,7 @@ gprtcuStatus trace_launch(const gprtcuLbvh *bvh, const uint32_t *tri_off, const 
   a.tm = TraceMeshes{tri_off, ray_off, meshes};
   a.rays = (const float4 *)rays;
   a.nrays = nrays;
-  a.lanes = lanes;
+  a.lanes = g.lanes;
   a.hits = (Hit *)hits;
   a.counter = counter;
   a.err = &hdr->status;
@@ -450,11 +429,11 @@ gprtcuStatus trace_launch(const gprtcuLbvh *bvh, const uint32_t *tri_off, const 
 #define GPRTCU_TRACE(K)                                                             \
   do {                                                                              \
     if (meshes > 1) {                                                               \
-      if (v8) K<true, true><<<grid, kTraceThreads, 0, stream>>>(a);                 \
-      else K<true, false><<<grid, kTraceThreads, 0, stream>>>(a);                   \
+      if (v8) K<true, true><<<g.ctas, kTraceThreads, 0, stream>>>(a);               \
+      else K<true, false><<<g.ctas, kTraceThreads, 0, stream>>>(a);                   \
     } else {                                                                        \
-      if (v8) K<false, true><<<grid, kTraceThreads, 0, stream>>>(a);                \
-      else K<false, false><<<grid, kTraceThreads, 0, stream>>>(a);                  \
+      if (v8) K<false, true><<<g.ctas, kTraceThreads, 0, stream>>>(a);                \
+      else K<false, false><<<g.ctas, kTraceThreads, 0, stream>>>(a);                  \
     }                                                                               \
   } while (0)
   if (any) GPRTCU_TRACE(k_trace_any);

@@ -118,3 +118,39 @@ def test_instance_node_alignment(cuda, anyhit):
         out.append((h.clone(), i.clone()))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
     assert int((out[0][1] >= 0).sum()) > 100
+
+
+@pytest.mark.parametrize("m", [1, 37, 4099, 151553])
+def test_prims_forms(cuda, m):
+    """Spheres and swept spheres: few to many rays, nodes on 16-byte
+    boundaries; against the oracle's search over every primitive where that is
+    small, else against the 32-byte form."""
+    import torch
+    from gprt_b200 import api
+    n = 300 if m < 5000 else 20000
+    rng = np.random.default_rng(m)
+    v = np.concatenate([rng.random((n + 1, 3)), rng.uniform(0.002, 0.02, (n + 1, 1))], 1).astype(np.float32)
+    idx = np.stack([np.arange(n), np.arange(n) + 1], 1).astype(np.uint32)
+    v[:, :3] = np.cumsum(np.vstack([v[:1, :3], rng.normal(0, 0.03, (n, 3))]), 0) % 1.0
+    vt, it = torch.from_numpy(v.astype(np.float32)).cuda(), torch.from_numpy(idx.view(np.int32)).cuda()
+    rays_h = scenes.rays(m, seed=m)
+    rays = torch.from_numpy(rays_h).cuda()
+    for kind in (0, 1):
+        out = []
+        for shift in (0, 16):
+            b = api.Lbvh(n)
+            _shift_nodes(b, shift)
+            api.lbvh_build_boxes(api.sphere_bounds(vt[:n]) if kind == 0 else api.lss_bounds(vt, it), b)
+            u = torch.zeros(m, device="cuda")
+            h = api.trace_spheres(b, vt[:n], rays, u=u) if kind == 0 else api.trace_lss(b, vt, it, rays, u=u)
+            a = api.trace_spheres(b, vt[:n], rays, anyhit=True) if kind == 0 else api.trace_lss(b, vt, it, rays,
+                                                                                              anyhit=True)
+            assert torch.equal(a[:, 0] == -1, h[:, 0] == -1)
+            out.append((api.hits_numpy(h), u.cpu().numpy()))
+        (h0, u0), (h1, u1) = out
+        assert np.array_equal(h0["prim"], h1["prim"]) and np.array_equal(h0["t"].view(np.uint32),
+                                                                        h1["t"].view(np.uint32))
+        assert np.array_equal(u0.view(np.uint32), u1.view(np.uint32))
+        if n == 300:
+            e = oracle.trace_user_brute(kind, v[:n] if kind == 0 else v, rays_h, *(() if kind == 0 else (idx,)))
+            assert np.array_equal(h0["prim"], e["prim"])
