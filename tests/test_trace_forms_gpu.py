@@ -154,3 +154,70 @@ def test_prims_forms(cuda, m):
         if n == 300:
             e = oracle.trace_user_brute(kind, v[:n] if kind == 0 else v, rays_h, *(() if kind == 0 else (idx,)))
             assert np.array_equal(h0["prim"], e["prim"])
+
+
+@pytest.mark.parametrize("stride", [32, 36, 48])
+@pytest.mark.parametrize("shift", [0, 16])
+def test_solid_forms(cuda, stride, shift):
+    """Point location with every cell type, index records on 16-byte
+    boundaries or not, nodes likewise, and few to many points: the answers of
+    the default layout, a sample of them equal to the oracle's search."""
+    import torch
+    from gprt_b200 import api
+    verts, idx, types = scenes.solid_grid(7, seed=2)
+    n = types.size
+    wide = np.full((n, stride // 4), 0xFFFFFFFF, np.uint32)
+    wide[:, :8] = idx
+    vt, tt = torch.from_numpy(verts).cuda(), torch.from_numpy(types).cuda()
+    std = api.Solids(vt, torch.from_numpy(idx.view(np.int32)).cuda(), tt)
+    alt = api.Solids(vt, torch.from_numpy(wide.view(np.int32)).cuda(), tt)
+    alt.desc.indexStride = stride
+    for m in (1, 9, 70, 60001):
+        pts_h = np.random.default_rng(m).random((m, 4), dtype=np.float32) * 1.1 - 0.05
+        pts = torch.from_numpy(pts_h).cuda()
+        out = []
+        for sol, sh in ((std, 0), (alt, shift)):
+            b = api.Lbvh(n)
+            _shift_nodes(b, sh)
+            api.lbvh_build_boxes(api.solid_bounds(sol)[1], b)
+            out.append(api.locate_solid_points(b, sol, pts))
+        assert torch.equal(out[0][0], out[1][0])
+        assert torch.equal(out[0][1].view(torch.int32), out[1][1].view(torch.int32))
+        if m == 70:
+            ec, ek, er = oracle.solid_locate_brute(verts, idx, types, pts_h)
+            got = out[0][0].cpu().numpy().view(np.uint32)
+            assert np.array_equal(got[:, 0], ec) and np.array_equal(got[:, 1], ek)
+            assert np.array_equal(out[0][1].cpu().numpy().view(np.uint32), er.view(np.uint32))
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-6, 1e9, 1e18])
+def test_solid_degenerate_cells(cuda, scale):
+    """Cells on which the inversion misbehaves -- random vertices (tangled,
+    inverted), repeated and collinear ones, magnitudes at which products
+    overflow or vanish -- get the oracle's answers bit for bit."""
+    import torch
+    from gprt_b200 import api
+    rng = np.random.default_rng(5)
+    kinds = np.array([10, 14, 13, 12, 23], np.uint8)
+    n = 400
+    types = kinds[np.arange(n) % 5]
+    verts = np.concatenate([rng.random((8 * n, 3)), rng.normal(size=(8 * n, 1))], 1)
+    cells = verts.reshape(n, 8, 4)
+    cells[::7, 1] = cells[::7, 0]
+    cells[1::7, 2:, :3] = cells[1::7, :1, :3] + rng.random((len(cells[1::7]), 6, 1)) * (cells[1::7, 1:2, :3] -
+                                                                                      cells[1::7, :1, :3])
+    cells[2::7, :, 2] = 0.5
+    cells[3::7, :4] = np.round(cells[3::7, :4])
+    verts[:, :3] *= scale
+    verts = verts.astype(np.float32)
+    idx = np.arange(8 * n, dtype=np.uint32).reshape(n, 8)
+    pts = np.zeros((3000, 4), np.float32)
+    pts[:, :3] = rng.random((3000, 3)) * scale
+    pts[:200, :3] = verts[rng.choice(8 * n, 200), :3]
+    sol = api.Solids(torch.from_numpy(verts).cuda(), torch.from_numpy(idx.view(np.int32)).cuda(),
+                     torch.from_numpy(types).cuda())
+    hits, rstw = api.locate_solid_points(api.lbvh_build_boxes(api.solid_bounds(sol)[1]), sol, torch.from_numpy(pts).cuda())
+    ec, ek, er = oracle.solid_locate_brute(verts, idx, types, pts)
+    got = hits.cpu().numpy().view(np.uint32)
+    assert np.array_equal(got[:, 0], ec) and np.array_equal(got[:, 1], ek)
+    assert np.array_equal(rstw.cpu().numpy().view(np.uint32), er.view(np.uint32))
