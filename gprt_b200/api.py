@@ -569,8 +569,9 @@ def wide_decode(wide):
     torch.cuda.synchronize()
     cnt = int(wide.count.item())
     raw = wide.nodes[:cnt].cpu().numpy().view(np.uint8).reshape(cnt, 80)
+    raw[1::2] = np.roll(raw[1::2], -16, axis=1)  # an odd node's last 16-byte word comes first
     f = raw[:, 0:12].copy().view(np.float32).reshape(cnt, 3)
-    e = raw[:, 12:15].copy().view(np.int8).astype(np.int32)
+    e = raw[:, 12:15].astype(np.int32) - 127
     imask = raw[:, 15].astype(np.uint32)
     cb = raw[:, 16:20].copy().view(np.uint32).ravel()
     lb = raw[:, 20:24].copy().view(np.uint32).ravel()

@@ -132,14 +132,9 @@ __device__ __forceinline__ unsigned long long pk2(float a, float b) {
 __device__ __forceinline__ void up2(unsigned long long v, float &a, float &b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
-__device__ __forceinline__ unsigned long long fma2_rd(unsigned long long a, unsigned long long b, unsigned long long c) {
+__device__ __forceinline__ unsigned long long fma2_rn(unsigned long long a, unsigned long long b, unsigned long long c) {
   unsigned long long r;
-  asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ unsigned long long fma2_ru(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rp.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
 __device__ __forceinline__ unsigned long long add2_rn(unsigned long long a, unsigned long long b) {

@@ -7,8 +7,9 @@
 //
 // Node (80 bytes, five 16-byte loads):
 //   p.xyz      fp32 origin = min corner of the children's union box
-//   e.xyz      int8 scale exponents, scale s = 2^e per axis, chosen (in FP64)
-//              as the smallest power of two with 255 * s >= extent
+//   e.xyz      scale exponents + 127 in a byte each, scale s = 2^e per axis,
+//              chosen (in FP64) as the smallest power of two with 255 * s >=
+//              extent
 //   imask      bit c: child slot c is an inner node
 //   child_base first inner child's node index (inner children contiguous)
 //   leaf_base  first leaf child's index in the wide leaf array (contiguous)
@@ -25,11 +26,13 @@
 #include "lbvh.cuh"
 #include "rtmath.cuh"
 
+#include <type_traits>
+
 namespace gprtcu {
 
 struct __align__(16) WideNode {
   float px, py, pz;
-  int8_t ex, ey, ez;
+  uint8_t ex, ey, ez;
   uint8_t imask;
   uint32_t child_base;
   uint32_t leaf_base;
@@ -38,6 +41,17 @@ struct __align__(16) WideNode {
   uint8_t qhi[3][8];
 };
 static_assert(sizeof(WideNode) == 80, "80-byte wide node");
+
+// The five 16-byte words of a node in memory: an even node has words 0..4 in
+// order, an odd one word 4 first and then words 0..3, so that words (0, 1) and
+// (2, 3) of every node lie on 32-byte boundaries (80-byte nodes from a 32-byte
+// boundary on) and a node is three loads instead of five.  Lanes visit
+// different nodes, so L1 serves a load instruction one lane per cycle
+// whatever its width.
+__device__ __forceinline__ uint32_t wide_word(uint32_t node, uint32_t k) {
+  const uint32_t base = 5 * (node & 1u);  // position of word k within the pair of nodes
+  return (node & 1u) ? (k == 4 ? base : base + 1 + k) : k;
+}
 
 struct WorkItem {
   uint32_t mesh;
@@ -267,15 +281,15 @@ __global__ void __launch_bounds__(128) k_wide_level(const Bvh2Node *bvh2, const 
         qhi_w[k][h] |= qh[k] << sh;
       }
     }
-    // the 80-byte node as five 16-byte words (layout of WideNode)
-    uint4 *op = reinterpret_cast<uint4 *>(wnodes + idx);
-    op[0] = make_uint4(__float_as_uint(lo3[0]), __float_as_uint(lo3[1]), __float_as_uint(lo3[2]),
-                       (uint32_t)(uint8_t)e[0] | ((uint32_t)(uint8_t)e[1] << 8) | ((uint32_t)(uint8_t)e[2] << 16) |
-                           (imask << 24));
-    op[1] = make_uint4(child_base, leaf_base, meta_w[0], meta_w[1]);
-    op[2] = make_uint4(qlo_w[0][0], qlo_w[0][1], qlo_w[1][0], qlo_w[1][1]);
-    op[3] = make_uint4(qlo_w[2][0], qlo_w[2][1], qhi_w[0][0], qhi_w[0][1]);
-    op[4] = make_uint4(qhi_w[1][0], qhi_w[1][1], qhi_w[2][0], qhi_w[2][1]);
+    // the 80-byte node as five 16-byte words (layout of WideNode, wide_word)
+    uint4 *op = reinterpret_cast<uint4 *>(wnodes) + 5 * (size_t)(idx & ~1u);
+    op[wide_word(idx, 0)] = make_uint4(__float_as_uint(lo3[0]), __float_as_uint(lo3[1]), __float_as_uint(lo3[2]),
+                                       (uint32_t)(e[0] + 127) | ((uint32_t)(e[1] + 127) << 8) |
+                                           ((uint32_t)(e[2] + 127) << 16) | (imask << 24));
+    op[wide_word(idx, 1)] = make_uint4(child_base, leaf_base, meta_w[0], meta_w[1]);
+    op[wide_word(idx, 2)] = make_uint4(qlo_w[0][0], qlo_w[0][1], qlo_w[1][0], qlo_w[1][1]);
+    op[wide_word(idx, 3)] = make_uint4(qlo_w[2][0], qlo_w[2][1], qhi_w[0][0], qhi_w[0][1]);
+    op[wide_word(idx, 4)] = make_uint4(qhi_w[1][0], qhi_w[1][1], qhi_w[2][0], qhi_w[2][1]);
   }
 #undef CBOX
   // the last CTA to finish moves the level window to the appended items
@@ -299,12 +313,16 @@ __global__ void __launch_bounds__(128) k_wide_level(const Bvh2Node *bvh2, const 
 // ---------------------------------------------------------------------------
 constexpr int kWideThreads = 128;
 constexpr int kWideStack = 64;
-constexpr int kWideRefill = 8;
+constexpr int kWideCtas = 7;    // closest hit, per SM
+constexpr int kWideShared = 6;  // stack entries in shared memory
+constexpr int kWideRefill = 6;
 
-__device__ __forceinline__ float scale_of(int8_t e) { return __int_as_float(((int)e + 127) << 23); }
-// 2^15 x the node's quantisation step (infinity past the float range: the
-// axis then gives NaN and drops out of the box test, which stays conservative)
-__device__ __forceinline__ float scale15_of(int8_t e) { return __int_as_float(min((int)e + 142, 255) << 23); }
+// 2^15 x the quantisation step of axis 0..2 from a node's word of biased
+// exponents (infinity past the float range: the axis then gives NaN and drops
+// out of the box test, which stays conservative).
+template <int AXIS> __device__ __forceinline__ float scale15_of(uint32_t w) {
+  return __fmul_rn(__uint_as_float((AXIS == 0 ? w << 23 : (AXIS == 1 ? w << 15 : w << 7)) & 0x7F800000u), 32768.0f);
+}
 
 __device__ __forceinline__ void wide_leaf_test(const float4 *leaf, uint32_t i, const Ray &R, uint32_t &best,
                                                uint32_t &best_leaf, float &bt) {
@@ -389,32 +407,55 @@ __device__ __forceinline__ bool wide_take_ray(bool &active, bool &drained, uint3
 
 // One node step: the ray is moved into the node's quantised frame once, the
 // eight child boxes are tested two at a time with packed f32x2 arithmetic
-// (byte decode, directed-rounding slab FMAs, the 2^-18 widening) and
-// three-input min/max (68.7 -> 60.7 ms on the 134M-ray workload against the
-// scalar loop).  A plane byte q is decoded by one byte permute into the float
-// v = 1 + q 2^-15; with M = 2^15 x the step in t and the plane offset moved
-// down (near planes) or up (far planes) by M in that direction of rounding,
-// one directed-rounding FMA v M + (offset - M) gives a value never inside
-// q x step + offset, without a separate bias subtraction (47.8 -> 47.2 ms).
-// Absent children are inverted boxes and need no test of their own.  With
-// NEAREST the nearest hit inner child is found inside the box loop (closest
-// hit: entering the lowest hit slot instead measured 40.3 against 22.7 ms on
-// 16.8M rays of one 16.8M-triangle mesh); without it the lowest hit inner
-// slot is entered (any hit: 16.8 against 17.7 ms on the same rays).
+// (byte decode, slab FMAs, the 2^-18 widening) and three-input min/max (68.7
+// -> 60.7 ms on 134 M rays over 16,384 meshes against the scalar loop).  A
+// plane byte q is decoded by one byte permute into the float v = 1 + q 2^-15;
+// with M = 2^15 x the step in t and the plane offset moved down (near planes)
+// or up (far planes) by M in that direction of rounding, one FMA v M + (offset
+// - M) gives q x step + offset without a separate bias subtraction (47.8 ->
+// 47.2 ms).  The FMA rounds once, to nearest: it is off by 2^-24 of its own
+// result, which the widening by 2^-18 covers (only the offset's error is not
+// relative to the result, hence its directed steps); packed FMAs with directed
+// rounding cost two scalar ones each.  Absent children are inverted boxes and
+// need no test of their own.  What bounds the step is the ALU pipe (75 % busy:
+// permutes, min/max, selects), so a child's test puts the sign of exit - entry
+// into the miss mask by one funnel shift instead of a compare and a predicated
+// OR, and the nearest hit inner child (NEAREST: entering the lowest hit slot
+// instead measured 40.3 against 22.7 ms on 16.8 M rays of one 16.8
+// M-triangle mesh) is one predicated integer min per child over the entry
+// distance's bits with the slot in the lowest three: 4.60 -> 4.33 ms on 4.0 M
+// rays of 4.2 M triangles.  Without NEAREST the lowest hit inner slot is
+// entered (any hit: 16.8 against 17.7 ms on the same rays).  An exit that
+// underflows to -0 counts as behind the ray.
 struct WideStep {
   uint32_t hm;  // slots whose box is hit
   uint32_t imask, child_base, leaf_base, meta_lo, meta_hi;
   int ns;  // nearest hit inner slot, -1 if none
 };
 
-template <bool NEAREST>
+// Words 2k and 2k + 1 of a node's first four (p on a 32-byte boundary when V8).
+template <bool V8> __device__ __forceinline__ void load_words(const uint4 *p, uint4 &a, uint4 &b) {
+  if constexpr (V8) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+        : "l"(p));
+  } else {
+    a = __ldg(p);
+    b = __ldg(p + 1);
+  }
+}
+
+template <bool NEAREST, bool V8>
 __device__ __forceinline__ WideStep wide_node_step(const WideNode *nodes, uint32_t node, const Ray &R, float bt) {
   WideStep S;
   const uint4 *np = reinterpret_cast<const uint4 *>(nodes + node);
-  const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
+  const uint32_t odd = node & 1u;
+  uint4 w0, w1, w2, w3;
+  load_words<V8>(np + odd, w0, w1);
+  load_words<V8>(np + odd + 2, w2, w3);
+  const uint4 w4 = __ldg(np + (odd ? 0 : 4));
   const float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
-  const float sx = scale15_of((int8_t)(w0.w & 0xFF)), sy = scale15_of((int8_t)((w0.w >> 8) & 0xFF)),
-              sz = scale15_of((int8_t)((w0.w >> 16) & 0xFF));
+  const float sx = scale15_of<0>(w0.w), sy = scale15_of<1>(w0.w), sz = scale15_of<2>(w0.w);
   S.imask = w0.w >> 24;
   S.child_base = w1.x;
   S.leaf_base = w1.y;
@@ -442,11 +483,12 @@ __device__ __forceinline__ WideStep wide_node_step(const WideNode *nodes, uint32
       qf[a][1] = pos ? qh[a][1] : ql[a][1];
     }
   }
-  uint32_t hm = 0;
-  float nt = __int_as_float(0x7f800000);
-  int ns = -1;
+  // The children from the last to the first: a miss puts the sign of (exit -
+  // entry) into the miss mask by one funnel shift.
+  uint32_t miss = 0;
+  float tn[8];
   {
-    const unsigned long long lo2 = pk2(kBoxLo, kBoxLo), hi2 = pk2(kBoxHi, kBoxHi);
+    const unsigned long long lo2 = pk2(kBoxLo, kBoxLo), hi2 = pk2(kBoxHi, kBoxHi), neg2 = pk2(-1.0f, -1.0f);
     unsigned long long B2[3], N2[3], F2[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -455,7 +497,7 @@ __device__ __forceinline__ WideStep wide_node_step(const WideNode *nodes, uint32
       F2[a] = pk2(Af[a], Af[a]);
     }
 #pragma unroll
-    for (int cp = 0; cp < 4; ++cp) {
+    for (int cp = 3; cp >= 0; --cp) {
       const int h = cp >> 1;
       const uint32_t s0 = 0x7604u | ((uint32_t)((2 * cp) & 3) << 4), s1 = 0x7604u | ((uint32_t)((2 * cp + 1) & 3) << 4);
       float n[2][3], f[2][3];
@@ -465,70 +507,88 @@ __device__ __forceinline__ WideStep wide_node_step(const WideNode *nodes, uint32
                                            __uint_as_float(__byte_perm(qn[a][h], 0x3F800000u, s1)));
         const unsigned long long qf2 = pk2(__uint_as_float(__byte_perm(qf[a][h], 0x3F800000u, s0)),
                                            __uint_as_float(__byte_perm(qf[a][h], 0x3F800000u, s1)));
-        up2(fma2_rd(qn2, B2[a], N2[a]), n[0][a], n[1][a]);
-        up2(fma2_ru(qf2, B2[a], F2[a]), f[0][a], f[1][a]);
+        up2(fma2_rn(qn2, B2[a], N2[a]), n[0][a], n[1][a]);
+        up2(fma2_rn(qf2, B2[a], F2[a]), f[0][a], f[1][a]);
       }
-      float tn[2], tf[2];
+      float tf[2];
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        tn[k] = fmaxf(max3f(n[k][0], n[k][1], n[k][2]), R.tmin);
+        tn[2 * cp + k] = fmaxf(max3f(n[k][0], n[k][1], n[k][2]), R.tmin);
         tf[k] = min3f(f[k][0], f[k][1], f[k][2]);
       }
-      up2(mul2_rn(pk2(tn[0], tn[1]), lo2), tn[0], tn[1]);
+      const unsigned long long e2 = mul2_rn(pk2(tn[2 * cp], tn[2 * cp + 1]), lo2);
+      up2(e2, tn[2 * cp], tn[2 * cp + 1]);
       up2(mul2_rn(pk2(tf[0], tf[1]), hi2), tf[0], tf[1]);
-      // the widened exit clamped by the best distance: one compare per child
-      // tests both (45.4 against 46.6 ms for two compares, exit clamped first)
+      // the widened exit clamped by the best distance: one test per child
       tf[0] = fminf(tf[0], bt);
       tf[1] = fminf(tf[1], bt);
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int c = 2 * cp + k;
-        const bool hit = tn[k] <= tf[k];
-        hm |= (uint32_t)hit << c;
-        if (NEAREST && hit && ((S.imask >> c) & 1u) && tn[k] < nt) {
-          nt = tn[k];
-          ns = c;
-        }
-      }
+      float d[2];
+      up2(fma2_rn(e2, neg2, pk2(tf[0], tf[1])), d[0], d[1]);
+      miss = __funnelshift_l(__float_as_uint(d[1]), miss, 1);
+      miss = __funnelshift_l(__float_as_uint(d[0]), miss, 1);
     }
   }
+  const uint32_t hm = ~miss & 0xFFu;
   S.hm = hm;
-  S.ns = NEAREST ? ns : ((hm & S.imask) ? __ffs(hm & S.imask) - 1 : -1);
+  const uint32_t inner = hm & S.imask;
+  if constexpr (NEAREST) {
+    // nearest hit inner child: entry distances (not negative, so their bits
+    // order as integers do) with the slot in the three lowest bits
+    uint32_t best = 0xFFFFFFFFu;
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (inner & (1u << c)) best = min(best, (__float_as_uint(tn[c]) & ~7u) | (uint32_t)c);
+    S.ns = inner ? (int)(best & 7u) : -1;
+  } else {
+    S.ns = inner ? __ffs(inner) - 1 : -1;
+  }
   return S;
 }
 
 // The next node: the nearest hit inner child is entered and the other hit
 // inner children are pushed as one entry {child_base, slot mask | inner mask
 // << 8} (a popped slot's node is child_base + the inner children below it);
-// with no inner child hit, the top entry's lowest slot is popped.  Returns
-// false when the traversal is over (or the stack overflowed: status 5).
-__device__ __forceinline__ bool wide_next(const WideStep &S, uint2 *stack, int &sp, uint32_t &node, uint32_t *err) {
+// with no inner child hit, the top entry's lowest slot is popped.  The top
+// entry stays in registers (slot mask zero: none), the next SHARED below it in
+// shared memory, the rest in local memory.  Returns false when the traversal
+// is over (or the stack overflowed: status 5).
+template <int SHARED>
+__device__ __forceinline__ bool wide_next(const WideStep &S, uint2 &top, uint2 *sh, uint2 *over, int &sp,
+                                          uint32_t &node, uint32_t *err) {
   if (S.ns >= 0) {
     const uint32_t rest = S.hm & S.imask & ~(1u << S.ns);
     if (rest) {
-      if (sp >= kWideStack) {
-        atomicCAS(err, 0u, 5u);  // traversal stack overflow
-        return false;
+      if (top.y & 0xFFu) {
+        if (sp < SHARED) sh[sp * kWideThreads] = top;
+        else if (sp < kWideStack) over[sp - SHARED] = top;
+        else {
+          atomicCAS(err, 0u, 5u);  // traversal stack overflow
+          return false;
+        }
+        ++sp;
       }
-      stack[sp++] = make_uint2(S.child_base, rest | (S.imask << 8));
+      top = make_uint2(S.child_base, rest | (S.imask << 8));
     }
     node = S.child_base + (uint32_t)__popc(S.imask & ((1u << S.ns) - 1u));
     return true;
   }
-  if (sp > 0) {
-    uint2 &top = stack[sp - 1];
-    const uint32_t c = __ffs(top.y & 0xFFu) - 1;
-    top.y &= ~(1u << c);
-    node = top.x + (uint32_t)__popc((top.y >> 8) & ((1u << c) - 1u));
-    if ((top.y & 0xFFu) == 0) --sp;
-    return true;
+  if (!(top.y & 0xFFu)) return false;
+  const uint32_t c = __ffs(top.y & 0xFFu) - 1;
+  node = top.x + (uint32_t)__popc((top.y >> 8) & ((1u << c) - 1u));
+  top.y &= ~(1u << c);
+  if (!(top.y & 0xFFu) && sp > 0) {
+    --sp;
+    top = sp < SHARED ? sh[sp * kWideThreads] : over[sp - SHARED];
   }
-  return false;
+  return true;
 }
 
 __device__ __forceinline__ uint32_t wide_leaf_meta(const WideStep &S, int c) {
   return ((c < 4 ? S.meta_lo : S.meta_hi) >> (8 * (c & 3))) & 0xFF;
 }
+
+// The top bits of a word's four bytes, in order.
+__device__ __forceinline__ uint32_t wide_msbs(uint32_t w) { return (((w >> 7) & 0x01010101u) * 0x01020408u) >> 24; }
 
 // A finished ray's record: the primitive id and, until k_wide_refine
 // replaces it by t, the leaf slot of the triangle hit.
@@ -597,7 +657,7 @@ __global__ void __launch_bounds__(kRefineThreads) k_wide_refine(const float4 *le
 // children test those triangles together, whatever slots they are in (testing
 // them inside the child loop ran each slot's test separately with few lanes
 // active), and the first hit ends the ray.
-template <bool BATCHED>
+template <bool BATCHED, bool V8>
 __global__ void __launch_bounds__(kWideThreads, 8)
     k_trace_wide_any(const WideNode *nodes, const float4 *leaf, const uint32_t *roots, const uint32_t *ray_off,
                      uint32_t meshes, const float4 *rays, uint64_t nrays, Hit *hits, unsigned long long *counter,
@@ -607,7 +667,9 @@ __global__ void __launch_bounds__(kWideThreads, 8)
   Ray R;
   uint32_t node = 0, best = kMiss, best_leaf = 0;
   float bt = 0.0f;
-  uint2 stack[kWideStack];  // {child_base, mask of inner-child ranks still to visit}
+  __shared__ uint2 s_stack[kWideShared][kWideThreads];
+  uint2 *const sh = &s_stack[0][threadIdx.x];
+  uint2 over[kWideStack - kWideShared], top = make_uint2(0u, 0u);
   uint32_t warp_mesh = 0;  // a mesh at or below every ray this warp will still take
   int sp = 0;
   while (true) {
@@ -615,15 +677,16 @@ __global__ void __launch_bounds__(kWideThreads, 8)
                                counter)) {
       best = kMiss;
       best_leaf = 0;
-      bt = R.tmax;
+      bt = __fadd_rn(R.tmax, 0.0f);  // never -0 (wide_node_step tests a sign)
       sp = 0;
+      top.y = 0;
     }
     if (!__any_sync(FULL_MASK, active)) {
       if (drained) break;
       continue;
     }
     if (!active) continue;
-    const WideStep S = wide_node_step<false>(nodes, node, R, bt);
+    const WideStep S = wide_node_step<false, V8>(nodes, node, R, bt);
     uint32_t leaf_hit = S.hm & ~S.imask;
     while (leaf_hit) {
       const int c = __ffs(leaf_hit) - 1;
@@ -631,95 +694,119 @@ __global__ void __launch_bounds__(kWideThreads, 8)
       const uint32_t meta = wide_leaf_meta(S, c);
       if (meta != 0xFF) wide_leaf_test(leaf, S.leaf_base + meta, R, best, best_leaf, bt);
     }
-    if (best != kMiss || !wide_next(S, stack, sp, node, err)) {
+    if (best != kMiss || !wide_next<kWideShared>(S, top, sh, over, sp, node, err)) {
       hits[r] = wide_result(best, best_leaf);
       active = false;
     }
   }
 }
 
-constexpr int kLeafFlush = 24;  // queued triangle tests that trigger a flush
-constexpr int kLeafQueue = 256;  // per warp: one node step adds at most 8 per lane; a step that would overflow flushes first
+constexpr int kWideFlush = 16;  // queued entries that trigger a flush
+constexpr int kWideSteps = 3;   // node steps between two looks at what else is to be done
+constexpr int kWideQueue = kWideFlush + 32 * kWideSteps;  // a step queues at most 32 entries
 
 // Closest hit: one lane per ray, and the triangle tests of the hit leaf
-// children are queued per warp in shared memory as (triangle slot, lane)
-// pairs instead of being run at once.  A node step hits about one leaf
-// triangle per 14 lanes, so running the tests at once kept ~2 of 32 lanes
-// busy for the length of a triangle test in most steps.  When kLeafFlush
-// tests are queued, all 32 lanes run them (the owner's ray comes by
-// shuffles and from shared memory) and fold each hit into the owner's best
-// (t, id) key with one shared-memory atomicMin; the owners then take the
-// key's t as their culling distance.  A lane whose traversal is over while tests of its ray are still
+// children are queued per warp in shared memory instead of being run at once
+// (a node step hits about one leaf triangle per 14 lanes, so running the tests
+// at once kept ~2 of 32 lanes busy for the length of a triangle test in most
+// steps).  A step's hit leaves are one entry, {leaf_base, hit slots | inner
+// mask << 8 | lane << 16}.  When kWideFlush entries are queued their tests are
+// listed and run by all 32 lanes (the owner's ray comes by shuffles and from
+// shared memory), each hit folded into the owner's best (t, id) key with one
+// shared-memory atomicMin; the owners then take the key's t as their culling
+// distance.  A lane whose traversal is over while tests of its ray are still
 // queued waits for the flush, which also runs when no lane of the warp
 // traverses any more, or when the waiting lanes and the idle ones add up to a
 // refill.  The closest (t, id) over all tested triangles is the same in any
 // order of tests, so the hits equal the immediate test's; the culling
-// distance only lags.  On the 134M-ray workload flush thresholds of 8, 12,
-// 16, 24, 32 and 64 tests measured 56.2 / 55.4 / 55.1 / 54.8 / 55.1 / 55.2
-// ms against 57.6 ms for the immediate tests (t still refined in the
-// traversal then).
-template <bool BATCHED>
-__global__ void __launch_bounds__(kWideThreads, 9)
+// distance only lags.
+// One entry per lane and step (placing every test by a prefix sum over the
+// lanes in every step took as long as the tests), kWideSteps steps between two
+// looks at flush, refill and finished rays, and 72 registers without spills:
+// 4.0 M rays on 4.2 M triangles 5.08 -> 4.30 ms with the changes to the step
+// above, 77.5 M rays over 4,096 meshes 28.6 -> 24.9 ms, 1,048,576 rays on
+// 262,144 triangles 1.58 -> 1.33 ms.  7 / 8 / 9 CTAs per SM (72 / 64 / 56
+// registers, the last spilling): 4.33 / 4.44 / 4.61 ms; 1 / 2 / 3 / 4 / 5 / 8
+// steps: 4.83 / 4.45 / 4.44 / 4.39 / 4.59 / 4.66 ms; flush at 10 / 16 / 24
+// entries: 4.63 / 4.60 / 4.69 ms; refill at 4 / 6 / 8 idle lanes: 4.30 / 4.30
+// / 4.37 ms, and 25.2 / 24.9 / 24.8 ms on the 4,096 meshes.
+template <bool BATCHED, bool V8>
+__global__ void __launch_bounds__(kWideThreads, kWideCtas)
     k_trace_wide_closest(const WideNode *nodes, const float4 *leaf, const uint32_t *roots, const uint32_t *ray_off,
                          uint32_t meshes, const float4 *rays, uint64_t nrays, Hit *hits,
                          unsigned long long *counter, uint32_t *err) {
-  __shared__ uint32_t s_qslot[kWideThreads / 32][kLeafQueue];
-  __shared__ uint8_t s_qlane[kWideThreads / 32][kLeafQueue];
+  __shared__ uint2 s_stack[kWideShared][kWideThreads];
+  __shared__ uint2 s_queue[kWideThreads / 32][kWideQueue];
+  __shared__ uint8_t s_list[kWideThreads / 32][256];  // tests of 32 entries: entry | slot << 5
   __shared__ unsigned long long s_best[kWideThreads / 32][32];
   __shared__ uint32_t s_bslot[kWideThreads / 32][32];
   // what only the flush and the final store read stays in shared memory, not
-  // in registers: 56 registers let 9 CTAs share an SM (47.8 -> 46.6 ms)
+  // in registers
   __shared__ float s_rs[kWideThreads / 32][4][32];  // Sx, Sy, Sz, tmax of each lane's ray
   __shared__ int s_rk[kWideThreads / 32][32];        // kx | ky << 2 | kz << 4
   __shared__ unsigned long long s_rid[kWideThreads / 32][32];  // ray index
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-  uint32_t *qslot = s_qslot[wq];
-  uint8_t *qlane = s_qlane[wq];
+  const uint32_t lt = (1u << lane) - 1u;
+  uint2 *queue = s_queue[wq];
+  uint8_t *list = s_list[wq];
   unsigned long long *sbest = s_best[wq];
   uint32_t *sbslot = s_bslot[wq];
-  bool active = false, drained = false, done = false, pending = false;
+  bool active = false, drained = false, walking = false, pending = false;
   uint64_t r = 0;
   Ray R;
   uint32_t node = 0;
   float bt = 0.0f;
-  uint2 stack[kWideStack];
+  uint2 *const sh = &s_stack[0][threadIdx.x];
+  uint2 over[kWideStack - kWideShared], top = make_uint2(0u, 0u);
   uint32_t warp_mesh = 0;
-  int sp = 0, nq = 0;  // nq: queued tests, the same on every lane
+  int sp = 0, nq = 0;  // nq: queued entries, the same on every lane
 
   // Runs the queued tests with all lanes (warp-uniform call).
   auto flush = [&]() {
     __syncwarp();
     for (int b = 0; b < nq; b += 32) {
-      const int e = b + lane;
-      const uint32_t slot = e < nq ? qslot[e] : kMiss;
-      const int o = e < nq ? qlane[e] : lane;
-      Ray Q;
-      Q.ox = __shfl_sync(FULL_MASK, R.ox, o);
-      Q.oy = __shfl_sync(FULL_MASK, R.oy, o);
-      Q.oz = __shfl_sync(FULL_MASK, R.oz, o);
-      Q.tmin = __shfl_sync(FULL_MASK, R.tmin, o);
-      Q.Sx = s_rs[wq][0][o];
-      Q.Sy = s_rs[wq][1][o];
-      Q.Sz = s_rs[wq][2][o];
-      Q.tmax = s_rs[wq][3][o];
-      const int k = s_rk[wq][o];
-      Q.kx = k & 3;
-      Q.ky = (k >> 2) & 3;
-      Q.kz = k >> 4;
-      unsigned long long key = ~0ull;
-      if (slot != kMiss) {
-        const float4 a = __ldg(leaf + 3 * (size_t)slot), bb = __ldg(leaf + 3 * (size_t)slot + 1),
-                     c = __ldg(leaf + 3 * (size_t)slot + 2);
-        const float v0[3] = {a.x, a.y, a.z}, v1[3] = {bb.x, bb.y, bb.z}, v2[3] = {c.x, c.y, c.z};
-        float t;
-        if (isect_tri(Q, v0, v1, v2, t)) {
-          key = ((unsigned long long)t_order(t) << 32) | __float_as_uint(a.w);
-          atomicMin(&sbest[o], key);
+      const uint2 v = b + lane < nq ? queue[b + lane] : make_uint2(0u, 0u);
+      uint32_t bits = v.y & 0xFFu;
+      const uint32_t cnt = __popc(bits), inc = warp_incl_scan(cnt, lane);
+      const int total = (int)__shfl_sync(FULL_MASK, inc, 31);
+      for (uint32_t k = inc - cnt; bits; bits &= bits - 1u) list[k++] = (uint8_t)(lane | ((__ffs(bits) - 1) << 5));
+      __syncwarp();
+      for (int k = 0; k < total; k += 32) {
+        const bool on = k + lane < total;
+        const uint32_t code = on ? list[k + lane] : (uint32_t)lane;
+        const uint32_t ex = __shfl_sync(FULL_MASK, v.x, code & 31u), ey = __shfl_sync(FULL_MASK, v.y, code & 31u);
+        const int o = on ? (int)(ey >> 16) : lane;
+        // a leaf's rank among the node's leaves: the slots below it that are
+        // not inner (empty slots come last)
+        const uint32_t slot = ex + (uint32_t)__popc(~(ey >> 8) & ((1u << (code >> 5)) - 1u));
+        Ray Q;
+        Q.ox = __shfl_sync(FULL_MASK, R.ox, o);
+        Q.oy = __shfl_sync(FULL_MASK, R.oy, o);
+        Q.oz = __shfl_sync(FULL_MASK, R.oz, o);
+        Q.tmin = __shfl_sync(FULL_MASK, R.tmin, o);
+        Q.Sx = s_rs[wq][0][o];
+        Q.Sy = s_rs[wq][1][o];
+        Q.Sz = s_rs[wq][2][o];
+        Q.tmax = s_rs[wq][3][o];
+        const int kk = s_rk[wq][o];
+        Q.kx = kk & 3;
+        Q.ky = (kk >> 2) & 3;
+        Q.kz = kk >> 4;
+        unsigned long long key = ~0ull;
+        if (on) {
+          const float4 a = __ldg(leaf + 3 * (size_t)slot), bb = __ldg(leaf + 3 * (size_t)slot + 1),
+                       c = __ldg(leaf + 3 * (size_t)slot + 2);
+          const float v0[3] = {a.x, a.y, a.z}, v1[3] = {bb.x, bb.y, bb.z}, v2[3] = {c.x, c.y, c.z};
+          float t;
+          if (isect_tri(Q, v0, v1, v2, t)) {
+            key = ((unsigned long long)t_order(t) << 32) | __float_as_uint(a.w);
+            atomicMin(&sbest[o], key);
+          }
         }
+        __syncwarp();
+        if (key != ~0ull && sbest[o] == key) sbslot[o] = slot;  // one winner per owner
+        __syncwarp();
       }
-      __syncwarp();
-      if (key != ~0ull && sbest[o] == key) sbslot[o] = slot;  // one winner per owner
-      __syncwarp();
     }
     if (pending) {
       bt = t_from_order((uint32_t)(sbest[lane] >> 32));
@@ -731,9 +818,10 @@ __global__ void __launch_bounds__(kWideThreads, 9)
   while (true) {
     if (wide_take_ray<BATCHED>(active, drained, warp_mesh, r, R, node, roots, ray_off, meshes, rays, nrays,
                                counter)) {
-      bt = R.tmax;
+      bt = __fadd_rn(R.tmax, 0.0f);  // never -0 (wide_node_step tests a sign)
       sp = 0;
-      done = false;
+      top.y = 0;
+      walking = true;
       sbest[lane] = ((unsigned long long)t_order(R.tmax) << 32) | kMiss;
       s_rs[wq][0][lane] = R.Sx;
       s_rs[wq][1][lane] = R.Sy;
@@ -746,47 +834,29 @@ __global__ void __launch_bounds__(kWideThreads, 9)
       if (drained) break;
       continue;
     }
-    uint32_t lh = 0, lbase = 0, mlo = 0, mhi = 0;
-    if (active && !done) {
-      const WideStep S = wide_node_step<true>(nodes, node, R, bt);
-      lh = S.hm & ~S.imask;
-      lbase = S.leaf_base;
-      mlo = S.meta_lo;
-      mhi = S.meta_hi;
-      done = !wide_next(S, stack, sp, node, err);
-    }
-    const int cnt = __popc(lh);
-    const int total = (int)__reduce_add_sync(FULL_MASK, (unsigned)cnt);
-    if (total) {
-      if (nq + total > kLeafQueue) flush();
-      int pos;
-      if (!__any_sync(FULL_MASK, cnt > 1)) {
-        pos = nq + __popc(__ballot_sync(FULL_MASK, cnt) & ((1u << lane) - 1u));
-      } else {
-        int inc = cnt;  // inclusive prefix of the counts over the lanes
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int v = __shfl_up_sync(FULL_MASK, inc, d);
-          if (lane >= d) inc += v;
-        }
-        pos = nq + inc - cnt;
+#pragma unroll 1
+    for (int step = 0; step < kWideSteps; ++step) {
+      uint32_t lh = 0, lbase = 0;
+      if (walking) {
+        const WideStep S = wide_node_step<true, V8>(nodes, node, R, bt);
+        lbase = S.leaf_base;
+        lh = S.hm & ~S.imask;
+        // an empty slot (meta 0xFF; only an infinite scale lets one pass the
+        // box test) is no leaf
+        if (lh) lh = (lh & ~(wide_msbs(S.meta_lo) | (wide_msbs(S.meta_hi) << 4))) | (S.imask << 8) | (lane << 16);
+        walking = wide_next<kWideShared>(S, top, sh, over, sp, node, err);
       }
-      while (lh) {
-        const int c = __ffs(lh) - 1;
-        lh &= lh - 1u;
-        const uint32_t meta = ((c < 4 ? mlo : mhi) >> (8 * (c & 3))) & 0xFF;
-        qslot[pos] = meta == 0xFF ? kMiss : lbase + meta;
-        qlane[pos] = (uint8_t)lane;
-        ++pos;
+      const unsigned m = __ballot_sync(FULL_MASK, lh != 0);
+      if (lh) {
+        queue[nq + __popc(m & lt)] = make_uint2(lbase, lh);
+        pending = true;
       }
-      if (cnt) pending = true;
-      nq += total;
+      nq += __popc(m);
     }
-    const unsigned waiting = __ballot_sync(FULL_MASK, done && pending);
-    const unsigned running = __ballot_sync(FULL_MASK, active && !done);
-    const unsigned idle = __ballot_sync(FULL_MASK, !active);
-    if (nq >= kLeafFlush || (waiting && (!running || __popc(waiting) + __popc(idle) >= kWideRefill))) flush();
-    if (active && done && !pending) {
+    const unsigned waiting = __ballot_sync(FULL_MASK, active && !walking && pending);
+    const unsigned running = __ballot_sync(FULL_MASK, walking);
+    if (nq >= kWideFlush || (waiting && (!running || 32 - __popc(running) >= kWideRefill))) flush();
+    if (active && !walking && !pending) {
       hits[s_rid[wq][lane]] = wide_result((uint32_t)sbest[lane], sbslot[lane]);
       active = false;
     }
@@ -879,22 +949,22 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuWideTrace(const gprtcuWideBvh *bvh, con
   ScratchHeader *hdr = (ScratchHeader *)scratch;
   unsigned long long *counter = reinterpret_cast<unsigned long long *>(&hdr->ticket[0]);
   GPRTCU_TRY(cudaMemsetAsync(scratch, 0, sizeof(ScratchHeader), stream));
-  // any hit: 64 registers, 8 CTAs of 128 threads per SM; closest hit: 56, 9
-  const int blocks = gprtcu_num_sms() * (anyHit ? 8 : 9);
+  // any hit: 64 registers, 8 CTAs of 128 threads per SM; closest hit: 72, 7
+  const int blocks = gprtcu_num_sms() * (anyHit ? 8 : kWideCtas);
   const uint64_t need = (numRays + kWideThreads - 1) / kWideThreads;
   const int grid = (int)(need < (uint64_t)blocks ? need : blocks);
-#define GPRTCU_WTRACE(K, B)                                                                                 \
-  K<B><<<grid, kWideThreads, 0, stream>>>((const WideNode *)bvh->nodes, (const float4 *)bvh->leafTris, bvh->roots, \
-                                          rayOffsets, numMeshes, (const float4 *)rays, numRays, (Hit *)hits,      \
-                                          counter, &hdr->status)
-  if (numMeshes > 1) {
-    if (anyHit) GPRTCU_WTRACE(k_trace_wide_any, true);
-    else GPRTCU_WTRACE(k_trace_wide_closest, true);
-  } else {
-    if (anyHit) GPRTCU_WTRACE(k_trace_wide_any, false);
-    else GPRTCU_WTRACE(k_trace_wide_closest, false);
-  }
-#undef GPRTCU_WTRACE
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, kWideThreads, 0, stream>>>((const WideNode *)bvh->nodes, (const float4 *)bvh->leafTris, bvh->roots,
+                                              rayOffsets, numMeshes, (const float4 *)rays, numRays, (Hit *)hits,
+                                              counter, &hdr->status);
+  };
+  auto pick = [&](auto v8) {
+    constexpr bool V = decltype(v8)::value;
+    if (numMeshes > 1) anyHit ? launch(k_trace_wide_any<true, V>) : launch(k_trace_wide_closest<true, V>);
+    else anyHit ? launch(k_trace_wide_any<false, V>) : launch(k_trace_wide_closest<false, V>);
+  };
+  if (((uintptr_t)bvh->nodes & 31) == 0) pick(std::true_type());
+  else pick(std::false_type());
   GPRTCU_TRY(cudaGetLastError());
   const uint64_t need_r = (numRays + kRefineThreads - 1) / kRefineThreads;
   const int grid_r = (int)(need_r < (uint64_t)gprtcu_num_sms() * 4 ? need_r : gprtcu_num_sms() * 4);

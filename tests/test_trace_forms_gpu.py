@@ -221,3 +221,29 @@ def test_solid_degenerate_cells(cuda, scale):
     got = hits.cpu().numpy().view(np.uint32)
     assert np.array_equal(got[:, 0], ec) and np.array_equal(got[:, 1], ek)
     assert np.array_equal(rstw.cpu().numpy().view(np.uint32), er.view(np.uint32))
+
+
+@pytest.mark.parametrize("shift", [0, 16, 32])
+@pytest.mark.parametrize("n,m", [(1, 5), (2, 40), (9, 100), (3000, 4099), (20000, 100003)])
+def test_wide_forms(cuda, n, m, shift):
+    """Quantised traversal with its nodes on 32-byte boundaries or only on
+    16-byte ones, from one triangle up, rays inside and outside the box: the
+    oracle's hits; occlusion likewise."""
+    import torch
+    from gprt_b200 import api
+    pos, tri = scenes.soup(n, seed=n, sigma=0.02 if n > 100 else 0.3)
+    rays_h = scenes.rays(m, seed=m + 1)
+    rays_h[m // 2:, :3] = np.random.default_rng(m).random((m - m // 2, 3), dtype=np.float32)
+    rays_h[::5, 3] = 0.25
+    rays_h[1::5, 7] = 1.5
+    rays = torch.from_numpy(rays_h).cuda()
+    b = api.lbvh_build_triangles(torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda())
+    w = api.WideBvh(n)
+    buf = torch.zeros(20 * n + 64, dtype=torch.int32, device="cuda")
+    w.nodes = buf[shift // 4:shift // 4 + 20 * n].view(n, 20)
+    w.desc.nodes = w.nodes.data_ptr()
+    api.wide_build(b, wide=w)
+    exp = _expect(pos, tri, rays_h)
+    assert _same(api.hits_numpy(api.wide_trace(w, rays)), exp)
+    anyh = api.hits_numpy(api.wide_trace(w, rays, anyhit=True))
+    assert np.array_equal(anyh["prim"] != 0xFFFFFFFF, exp["prim"] != 0xFFFFFFFF)
