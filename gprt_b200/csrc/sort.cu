@@ -53,6 +53,17 @@ const std::array<SortRunFn, kSortGridSize> &table_for(int slot) {
   }
 }
 
+SortSmallFn small_for(int slot) {
+  switch (slot) {
+    case 0: return kSortSmallK32;
+    case 1: return kSortSmallK32V32;
+    case 2: return kSortSmallK64;
+    case 3: return kSortSmallK64V32;
+    case 5: return kSortSmallK32V64;
+    default: return kSortSmallK64V64;
+  }
+}
+
 int grid_index(int rb, int tile, int warps) {
   for (int i = 0; i < kSortGridSize; ++i)
     if (kSortGrid[i].rb == rb && kSortGrid[i].tile == tile && kSortGrid[i].warps == warps) return i;
@@ -61,20 +72,31 @@ int grid_index(int rb, int tile, int warps) {
 
 // Shapes used until the tuner or the caller picks others, from sweeps of the
 // grid on B200 (uniform and Zipf(1.1) keys, 2^18 .. 2^28 elements): 8-bit
-// digits everywhere; for 32-bit keys with 32-bit payloads 6144-key tiles of 8
-// warps (73 KB of shared memory and 80 registers: three CTAs per SM; 2^28
-// Zipf pairs 5.76 ms against 5.95 for 8192-key tiles, which fit two); 32-bit
-// keys alone or with 64-bit payloads 8192-key tiles of 8 warps (2^28 Zipf
-// keys 4.66 ms against 4.81 at 6144); 64-bit keys with 32-bit payloads
-// 6144-key tiles of 8 warps (2^26 segmented (mesh, code) pairs of 44 bits:
-// 3.09 ms against 3.14 at 4096 and 3.80 at 8192), other 64-bit keys
-// 4096-key tiles of 8 warps; 2048-key tiles of 8 warps below 2^22 keys, where
-// there are too few large tiles to fill the SMs.
+// digits and 8 warps, and a tile that grows with n.  A pass over few tiles is
+// a chain of look-backs from tile to tile, so few large tiles beat many small
+// ones as soon as they fill most of the SMs (times of whole sorts in us):
+//   below 2^19 keys 2048-key tiles (2^18 u32 pairs: 57 at 2048, 59 at 4096, 66
+//     at 8192), below 2^20 4096-key ones (2^19 u64/u32 pairs: 100 / 90 / 100);
+//   while 8192-key tiles all fit on the GPU at once (two CTAs per SM, one
+//     where key and payload take 12 bytes or more) 8192 (2^20 u32 pairs: 93 /
+//     83 / 75; 2^21: 133 / 111 / 103; 2^20 u64/u32 pairs 137 / 116 / 111; 2^20
+//     u64 pairs 140 / 124 / 112);
+//   beyond, 6144-key tiles, of which three CTAs share an SM with 32-bit keys
+//     and payloads (2.8 M u32 pairs: 156 / 133 / 121 at 6144 / 135 at 8192;
+//     2^28 Zipf pairs 5.76 ms against 5.95 at 8192; 2^26 segmented u64/u32
+//     pairs of 44 bits 3.09 ms against 3.14 at 4096; 10^8 u64 keys 4.56 ms
+//     against 5.00 at 4096), except u32 keys alone 8192 (2^28 Zipf keys 4.66 ms
+//     against 4.81) and u64 pairs 4096 with 16 warps (4.2 M: 349 against 384
+//     with 8 warps) and from 2^23 on 8192 with 16 warps (10^8: 7.13 ms against
+//     7.38 at 4096 and 8.03 at 6144).
 int default_index(int slot, uint64_t n) {
-  if (n < (1ull << 22)) return grid_index(8, 2048, 8);
-  if (slot == 1 || slot == 3) return grid_index(8, 6144, 8);
-  if (slot == 0 || slot == 5) return grid_index(8, 8192, 8);
-  return grid_index(8, 4096, 8);
+  if (n < (1ull << 19)) return grid_index(8, 2048, 8);
+  if (n < (1ull << 20)) return grid_index(8, 4096, 8);
+  const uint64_t per_sm = slot <= 2 ? 2 : 1;  // 8192-key CTAs that share an SM
+  if (n <= per_sm * (uint64_t)gprtcu_num_sms() * 8192) return grid_index(8, 8192, 8);
+  if (slot == 0) return grid_index(8, 8192, 8);
+  if (slot == 4) return n < (1ull << 23) ? grid_index(8, 4096, 16) : grid_index(8, 8192, 16);
+  return grid_index(8, 6144, 8);
 }
 
 std::atomic<int> g_active[kTypeSlots] = {{-1}, {-1}, {-1}, {-1}, {-1}, {-1}};
@@ -94,11 +116,8 @@ SortLayout sort_layout(uint64_t n, int kw, int vw, int begin_bit, int end_bit, c
   SortLayout L;
   L.tiles = (n + s.tile - 1) / s.tile;
   L.passes = (end_bit - begin_bit + s.rb - 1) / s.rb;
+  // what starts as zero first (one fill), then the ping-pong buffers
   size_t off = sizeof(SortHeader);
-  L.keys_alt = off;
-  off += gprtcu_align256((size_t)n * kw);
-  L.vals_alt = off;
-  off += gprtcu_align256((size_t)n * vw);
   L.hist = off;
   off += gprtcu_align256((size_t)SORT_MAX_PASSES * 256 * 4);
   L.trivial = off;
@@ -106,6 +125,10 @@ SortLayout sort_layout(uint64_t n, int kw, int vw, int begin_bit, int end_bit, c
   L.status = off;
   // look-back words: 32-bit, or 64-bit once n needs more than 30 value bits
   off += gprtcu_align256((size_t)2 * L.tiles * (1u << s.rb) * (n > (uint64_t)LB_VALUE ? 8 : 4));
+  L.keys_alt = off;
+  off += gprtcu_align256((size_t)n * kw);
+  L.vals_alt = off;
+  off += gprtcu_align256((size_t)n * vw);
   L.total = off;
   return L;
 }
@@ -124,8 +147,13 @@ size_t scratch_any_shape(uint64_t n, int kw, int vw) {
   return m;
 }
 
+// index: a shape of the grid, or -1 for the default, which for few keys is one
+// CTA instead of a shape (not with a test hook or another ranking set: those
+// are of the passes).
 gprtcuStatus sort_dispatch(int slot, int index, void *keys, void *vals, uint64_t n, int kw, int vw, int begin_bit,
                            int end_bit, void *scratch, size_t scratch_bytes, cudaStream_t stream) {
+  const bool small = index < 0 && n > 1 && n <= kSortSmallMax && g_sort_skip_tile < 0 && g_sort_ranking == 0;
+  if (index < 0) index = default_index(slot, n);
   if (!keys && n) return GPRTCU_ERR_INVALID_ARG;
   if (vw && !vals && n) return GPRTCU_ERR_INVALID_ARG;
   if (begin_bit < 0 || end_bit > 8 * kw || begin_bit >= end_bit) return GPRTCU_ERR_INVALID_ARG;
@@ -136,9 +164,11 @@ gprtcuStatus sort_dispatch(int slot, int index, void *keys, void *vals, uint64_t
   SortLayout L = sort_layout(n, kw, vw, begin_bit, end_bit, shape);
   if (scratch_bytes < L.total) return GPRTCU_ERR_SCRATCH_TOO_SMALL;
   char *s = (char *)scratch;
-  // the header (its status word first) is valid after every call, even one
-  // with nothing to sort: callers such as the LBVH build read it
-  GPRTCU_TRY(cudaMemsetAsync(s, 0, sizeof(SortHeader), stream));
+  // The header (its status word first) is valid after every call, even one
+  // with nothing to sort: callers such as the LBVH build read it.  One fill
+  // zeroes it with the histograms, trivial flags and both look-back regions
+  // (the one-CTA sort writes the header itself).
+  if (!small) GPRTCU_TRY(cudaMemsetAsync(s, 0, n <= 1 ? sizeof(SortHeader) : L.keys_alt, stream));
   if (n <= 1) return GPRTCU_OK;
   SortArgs a;
   a.keys = keys;
@@ -159,15 +189,14 @@ gprtcuStatus sort_dispatch(int slot, int index, void *keys, void *vals, uint64_t
   a.pf_tiles = 0;
   a.use_bulk = ((((uintptr_t)keys) | ((uintptr_t)a.keys_alt)) & 15) == 0;
   a.sms = gprtcu_num_sms();
-  // Zero: histograms, trivial flags, both look-back regions.
-  GPRTCU_TRY(cudaMemsetAsync(s + L.hist, 0, L.total - L.hist, stream));
+  if (small) return small_for(slot)(a, stream);
   return table_for(slot)[index](a, stream);
 }
 
 gprtcuStatus sort_entry(void *keys, void *vals, uint64_t n, int kw, int vw, int begin_bit, int end_bit,
                         void *scratch, size_t scratch_bytes, gprtcuStream stream) {
   const int slot = type_slot(kw, vw);
-  return sort_dispatch(slot, active_index(slot, n), keys, vals, n, kw, vw, begin_bit, end_bit, scratch, scratch_bytes,
+  return sort_dispatch(slot, g_active[slot].load(std::memory_order_relaxed), keys, vals, n, kw, vw, begin_bit, end_bit, scratch, scratch_bytes,
                        (cudaStream_t)stream);
 }
 

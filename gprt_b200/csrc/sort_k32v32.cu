@@ -4,4 +4,5 @@
 namespace gprtcu {
 const std::array<SortRunFn, kSortGridSize> kSortTableK32V32 =
     make_sort_table<uint32_t, uint32_t>(std::make_index_sequence<kSortGridSize>{});
+const SortSmallFn kSortSmallK32V32 = &sort_small_run<uint32_t, uint32_t>;
 }  // namespace gprtcu

@@ -4,4 +4,5 @@
 namespace gprtcu {
 const std::array<SortRunFn, kSortGridSize> kSortTableK32V64 =
     make_sort_table<uint32_t, uint64_t>(std::make_index_sequence<kSortGridSize>{});
+const SortSmallFn kSortSmallK32V64 = &sort_small_run<uint32_t, uint64_t>;
 }  // namespace gprtcu

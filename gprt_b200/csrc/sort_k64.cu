@@ -4,4 +4,5 @@
 namespace gprtcu {
 const std::array<SortRunFn, kSortGridSize> kSortTableK64 =
     make_sort_table<uint64_t, char>(std::make_index_sequence<kSortGridSize>{});
+const SortSmallFn kSortSmallK64 = &sort_small_run<uint64_t, char>;
 }  // namespace gprtcu

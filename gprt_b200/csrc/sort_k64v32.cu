@@ -4,4 +4,5 @@
 namespace gprtcu {
 const std::array<SortRunFn, kSortGridSize> kSortTableK64V32 =
     make_sort_table<uint64_t, uint32_t>(std::make_index_sequence<kSortGridSize>{});
+const SortSmallFn kSortSmallK64V32 = &sort_small_run<uint64_t, uint32_t>;
 }  // namespace gprtcu

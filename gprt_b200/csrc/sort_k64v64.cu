@@ -4,4 +4,5 @@
 namespace gprtcu {
 const std::array<SortRunFn, kSortGridSize> kSortTableK64V64 =
     make_sort_table<uint64_t, uint64_t>(std::make_index_sequence<kSortGridSize>{});
+const SortSmallFn kSortSmallK64V64 = &sort_small_run<uint64_t, uint64_t>;
 }  // namespace gprtcu

@@ -951,6 +951,118 @@ gprtcuStatus sort_run(const SortArgs &a, cudaStream_t stream) {
   return GPRTCU_OK;
 }
 
+// ---------------------------------------------------------------------------
+// 3. a few thousand keys in one CTA
+// ---------------------------------------------------------------------------
+// Below kSortSmallMax keys the passes above are launches of a few tiles each:
+// ten launches, 40 to 45 us, for work of a few microseconds.  Here one CTA
+// holds keys and payloads in shared memory and sorts a 16-bit permutation of
+// them digit by digit: the warp's rows are ranked by leader tables as in
+// k_sort_pass8, warp counts become first slots by one scan, and the keys and
+// payloads move once, at the end.  Slots past n hold all-ones keys, which
+// stay last.  A chain of a few dependent shared-memory steps per row and pass
+// bounds it.  Whole sorts of 1,501 / 4,096 / 8,192 u32 pairs by 30 bits: 50 /
+// 41 / 42 -> 15 / 18 / 25 us; u64 pairs by 64 bits: 83 / 69 / 69 -> 21 / 30 /
+// 44 us.
+constexpr uint32_t kSortSmallMax = 8192;
+constexpr int kSortSmallThreads = 1024;
+constexpr int kSortSmallWarps = kSortSmallThreads / 32;
+
+template <typename K, typename V> struct SmallCfg {
+  static constexpr size_t VB = sizeof(V) > 1 ? sizeof(V) : 0;
+  static constexpr size_t TBL = (size_t)kSortSmallWarps * 256 * 4, LEAD = (size_t)kSortSmallWarps * 512;
+  // slots: a multiple of the CTA's threads
+  static size_t smem(uint32_t slots) { return TBL + LEAD + slots * (sizeof(K) + VB + 4); }
+};
+
+template <typename K, typename V>
+__global__ void __launch_bounds__(kSortSmallThreads, 1) k_sort_small(K *keys, V *vals, uint32_t n, int begin_bit,
+                                                                     int end_bit, SortHeader *hdr) {
+  using C = SmallCfg<K, V>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ uint32_t s_tmp[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t rows = (n + kSortSmallThreads - 1) / kSortSmallThreads, slots = rows * kSortSmallThreads;
+  uint32_t *s_cnt = reinterpret_cast<uint32_t *>(smem);  // [warps][256]
+  uint8_t *s_lead = smem + C::TBL;
+  K *s_keys = reinterpret_cast<K *>(smem + C::TBL + C::LEAD);
+  V *s_vals = reinterpret_cast<V *>(smem + C::TBL + C::LEAD + slots * sizeof(K));
+  uint16_t *s_perm = reinterpret_cast<uint16_t *>(smem + C::TBL + C::LEAD + slots * (sizeof(K) + C::VB));
+  uint16_t *cur = s_perm, *nxt = s_perm + slots;
+  for (uint32_t i = tid; i < slots; i += kSortSmallThreads) {
+    s_keys[i] = i < n ? keys[i] : ~(K)0;
+    if constexpr (C::VB > 0)
+      if (i < n) s_vals[i] = vals[i];
+    cur[i] = (uint16_t)i;
+  }
+  if (tid < (int)(sizeof(SortHeader) / 4)) reinterpret_cast<uint32_t *>(hdr)[tid] = 0;
+  uint32_t *wc = s_cnt + warp * 256;
+  uint8_t *wl = s_lead + warp * 512;
+  const uint32_t lt = (1u << lane) - 1u, first = (uint32_t)warp * rows * 32 + lane;
+  for (int shift = begin_bit; shift < end_bit; shift += 8) {
+    const uint32_t mask = (1u << min(8, end_bit - shift)) - 1u;
+    for (int i = lane; i < 256; i += 32) wc[i] = 0;
+    __syncthreads();  // the permutation (and the keys, the first time) complete
+    uint32_t rank[kSortSmallMax / kSortSmallThreads];
+#pragma unroll
+    for (uint32_t r = 0; r < kSortSmallMax / kSortSmallThreads; ++r) {
+      if (r >= rows) break;
+      const uint32_t d = digit_of(s_keys[cur[first + 32 * r]], shift, mask);
+      uint8_t *t = wl + (r & 1u) * 256;
+      t[d] = (uint8_t)lane;
+      const uint32_t base = wc[d];
+      __syncwarp();
+      const uint32_t peers = warp_peers_p<5>(t[d]);
+      __syncwarp();
+      wc[d] = base + __popc(peers);  // every peer stores the same count
+      __syncwarp();
+      rank[r] = base + __popc(peers & lt);
+    }
+    __syncthreads();
+    uint32_t total = 0;
+    if (tid < 256)
+#pragma unroll 8
+      for (int w = 0; w < kSortSmallWarps; ++w) total += s_cnt[w * 256 + tid];
+    uint32_t run = block_excl_scan_digits<256>(total, s_tmp);
+    if (tid < 256)
+#pragma unroll 8
+      for (int w = 0; w < kSortSmallWarps; ++w) {
+        const uint32_t c = s_cnt[w * 256 + tid];
+        s_cnt[w * 256 + tid] = run;
+        run += c;
+      }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t r = 0; r < kSortSmallMax / kSortSmallThreads; ++r) {
+      if (r >= rows) break;
+      const uint16_t src = cur[first + 32 * r];
+      nxt[wc[digit_of(s_keys[src], shift, mask)] + rank[r]] = src;
+    }
+    __syncthreads();
+    uint16_t *x = cur;
+    cur = nxt;
+    nxt = x;
+  }
+  for (uint32_t i = tid; i < n; i += kSortSmallThreads) {
+    const uint32_t src = cur[i];
+    keys[i] = s_keys[src];
+    if constexpr (C::VB > 0) vals[i] = s_vals[src];
+  }
+}
+
+using SortSmallFn = gprtcuStatus (*)(const SortArgs &, cudaStream_t);
+template <typename K, typename V> gprtcuStatus sort_small_run(const SortArgs &a, cudaStream_t stream) {
+  const uint32_t n = (uint32_t)a.n;
+  const uint32_t slots = (n + kSortSmallThreads - 1) / kSortSmallThreads * kSortSmallThreads;
+  const size_t smem = SmallCfg<K, V>::smem(slots);
+  GPRTCU_TRY(cudaFuncSetAttribute(k_sort_small<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)SmallCfg<K, V>::smem(kSortSmallMax)));
+  k_sort_small<K, V><<<1, kSortSmallThreads, smem, stream>>>(static_cast<K *>(a.keys), static_cast<V *>(a.vals), n,
+                                                             a.begin_bit, a.end_bit, a.hdr);
+  GPRTCU_TRY(cudaGetLastError());
+  return GPRTCU_OK;
+}
+
 template <typename K, typename V, size_t... I>
 constexpr std::array<SortRunFn, sizeof...(I)> make_sort_table(std::index_sequence<I...>) {
   return {{&sort_run<K, V, kSortGrid[I].rb, kSortGrid[I].warps, kSortGrid[I].tile / (32 * kSortGrid[I].warps)>...}};
@@ -964,5 +1076,7 @@ extern const std::array<SortRunFn, kSortGridSize> kSortTableK32V64;
 extern const std::array<SortRunFn, kSortGridSize> kSortTableK64;
 extern const std::array<SortRunFn, kSortGridSize> kSortTableK64V32;
 extern const std::array<SortRunFn, kSortGridSize> kSortTableK64V64;
+extern const SortSmallFn kSortSmallK32, kSortSmallK32V32, kSortSmallK32V64, kSortSmallK64, kSortSmallK64V32,
+    kSortSmallK64V64;
 
 }  // namespace gprtcu
