@@ -313,28 +313,15 @@ __global__ void __launch_bounds__(128) k_wide_level(const Bvh2Node *bvh2, const 
 // ---------------------------------------------------------------------------
 constexpr int kWideThreads = 128;
 constexpr int kWideStack = 64;
-constexpr int kWideCtas = 7;    // closest hit, per SM
+constexpr int kWideCtas = 7;    // per SM: 72 registers
 constexpr int kWideShared = 6;  // stack entries in shared memory
 constexpr int kWideRefill = 6;
 
-// 2^15 x the quantisation step of axis 0..2 from a node's word of biased
+// 2^16 x the quantisation step of axis 0..2 from a node's word of biased
 // exponents (infinity past the float range: the axis then gives NaN and drops
 // out of the box test, which stays conservative).
-template <int AXIS> __device__ __forceinline__ float scale15_of(uint32_t w) {
-  return __fmul_rn(__uint_as_float((AXIS == 0 ? w << 23 : (AXIS == 1 ? w << 15 : w << 7)) & 0x7F800000u), 32768.0f);
-}
-
-__device__ __forceinline__ void wide_leaf_test(const float4 *leaf, uint32_t i, const Ray &R, uint32_t &best,
-                                               uint32_t &best_leaf, float &bt) {
-  const float4 a = __ldg(leaf + 3 * (size_t)i), b = __ldg(leaf + 3 * (size_t)i + 1), c = __ldg(leaf + 3 * (size_t)i + 2);
-  const float v0[3] = {a.x, a.y, a.z}, v1[3] = {b.x, b.y, b.z}, v2[3] = {c.x, c.y, c.z};
-  const uint32_t id = __float_as_uint(a.w);
-  float t;
-  if (isect_tri(R, v0, v1, v2, t) && (best == kMiss || t < bt || (t == bt && id < best))) {
-    best = id;
-    best_leaf = i;
-    bt = t;
-  }
+template <int AXIS> __device__ __forceinline__ float scale16_of(uint32_t w) {
+  return __fmul_rn(__uint_as_float((AXIS == 0 ? w << 23 : (AXIS == 1 ? w << 15 : w << 7)) & 0x7F800000u), 65536.0f);
 }
 
 // Largest m < meshes with off[m] <= r, given off[m0] <= r: gallop upward
@@ -409,8 +396,8 @@ __device__ __forceinline__ bool wide_take_ray(bool &active, bool &drained, uint3
 // eight child boxes are tested two at a time with packed f32x2 arithmetic
 // (byte decode, slab FMAs, the 2^-18 widening) and three-input min/max (68.7
 // -> 60.7 ms on 134 M rays over 16,384 meshes against the scalar loop).  A
-// plane byte q is decoded by one byte permute into the float v = 1 + q 2^-15;
-// with M = 2^15 x the step in t and the plane offset moved down (near planes)
+// plane byte q is decoded by one instruction into the float v = 1 + q 2^-16;
+// with M = 2^16 x the step in t and the plane offset moved down (near planes)
 // or up (far planes) by M in that direction of rounding, one FMA v M + (offset
 // - M) gives q x step + offset without a separate bias subtraction (47.8 ->
 // 47.2 ms).  The FMA rounds once, to nearest: it is off by 2^-24 of its own
@@ -418,7 +405,9 @@ __device__ __forceinline__ bool wide_take_ray(bool &active, bool &drained, uint3
 // relative to the result, hence its directed steps); packed FMAs with directed
 // rounding cost two scalar ones each.  Absent children are inverted boxes and
 // need no test of their own.  What bounds the step is the ALU pipe (75 % busy:
-// permutes, min/max, selects), so a child's test puts the sign of exit - entry
+// byte permutes, min/max, selects), so the bytes are decoded on the FMA pipe
+// (wide_plane: 4.29 -> 4.02 ms on 4.0 M rays of 4.2 M triangles, 24.9 -> 24.2
+// ms on 77.5 M rays over 4,096 meshes), a child's test puts the sign of exit - entry
 // into the miss mask by one funnel shift instead of a compare and a predicated
 // OR, and the nearest hit inner child (NEAREST: entering the lowest hit slot
 // instead measured 40.3 against 22.7 ms on 16.8 M rays of one 16.8
@@ -445,6 +434,13 @@ template <bool V8> __device__ __forceinline__ void load_words(const uint4 *p, ui
   }
 }
 
+// Plane byte c of a word as the float 1 + q 2^-16: the dot product with one
+// byte 128 added to the bits of 1.0.  It runs on the FMA pipe, where a byte
+// permute is one of the ALU pipe's 250 instructions per step.
+__device__ __forceinline__ float wide_plane(uint32_t q, int c) {
+  return __uint_as_float(__dp4a(q, 128u << (8 * (c & 3)), 0x3F800000u));
+}
+
 template <bool NEAREST, bool V8>
 __device__ __forceinline__ WideStep wide_node_step(const WideNode *nodes, uint32_t node, const Ray &R, float bt) {
   WideStep S;
@@ -455,7 +451,7 @@ __device__ __forceinline__ WideStep wide_node_step(const WideNode *nodes, uint32
   load_words<V8>(np + odd + 2, w2, w3);
   const uint4 w4 = __ldg(np + (odd ? 0 : 4));
   const float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
-  const float sx = scale15_of<0>(w0.w), sy = scale15_of<1>(w0.w), sz = scale15_of<2>(w0.w);
+  const float sx = scale16_of<0>(w0.w), sy = scale16_of<1>(w0.w), sz = scale16_of<2>(w0.w);
   S.imask = w0.w >> 24;
   S.child_base = w1.x;
   S.leaf_base = w1.y;
@@ -474,7 +470,7 @@ __device__ __forceinline__ WideStep wide_node_step(const WideNode *nodes, uint32
       const bool pos = !(ia[a] < 0.0f);
       An[a] = __fmul_rd(pos ? dlo : dhi, ia[a]);
       Af[a] = __fmul_ru(pos ? dhi : dlo, ia[a]);
-      Bq[a] = __fmul_rn(sa[a], ia[a]);  // M: 2^15 x the step in t (exactly 2^15 x the rounded step)
+      Bq[a] = __fmul_rn(sa[a], ia[a]);  // M: 2^16 x the step in t (exactly 2^16 x the rounded step)
       An[a] = __fsub_rd(An[a], Bq[a]);
       Af[a] = __fsub_ru(Af[a], Bq[a]);
       qn[a][0] = pos ? ql[a][0] : qh[a][0];
@@ -499,14 +495,11 @@ __device__ __forceinline__ WideStep wide_node_step(const WideNode *nodes, uint32
 #pragma unroll
     for (int cp = 3; cp >= 0; --cp) {
       const int h = cp >> 1;
-      const uint32_t s0 = 0x7604u | ((uint32_t)((2 * cp) & 3) << 4), s1 = 0x7604u | ((uint32_t)((2 * cp + 1) & 3) << 4);
       float n[2][3], f[2][3];
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        const unsigned long long qn2 = pk2(__uint_as_float(__byte_perm(qn[a][h], 0x3F800000u, s0)),
-                                           __uint_as_float(__byte_perm(qn[a][h], 0x3F800000u, s1)));
-        const unsigned long long qf2 = pk2(__uint_as_float(__byte_perm(qf[a][h], 0x3F800000u, s0)),
-                                           __uint_as_float(__byte_perm(qf[a][h], 0x3F800000u, s1)));
+        const unsigned long long qn2 = pk2(wide_plane(qn[a][h], 2 * cp), wide_plane(qn[a][h], 2 * cp + 1));
+        const unsigned long long qf2 = pk2(wide_plane(qf[a][h], 2 * cp), wide_plane(qf[a][h], 2 * cp + 1));
         up2(fma2_rn(qn2, B2[a], N2[a]), n[0][a], n[1][a]);
         up2(fma2_rn(qf2, B2[a], F2[a]), f[0][a], f[1][a]);
       }
@@ -583,10 +576,6 @@ __device__ __forceinline__ bool wide_next(const WideStep &S, uint2 &top, uint2 *
   return true;
 }
 
-__device__ __forceinline__ uint32_t wide_leaf_meta(const WideStep &S, int c) {
-  return ((c < 4 ? S.meta_lo : S.meta_hi) >> (8 * (c & 3))) & 0xFF;
-}
-
 // The top bits of a word's four bytes, in order.
 __device__ __forceinline__ uint32_t wide_msbs(uint32_t w) { return (((w >> 7) & 0x01010101u) * 0x01020408u) >> 24; }
 
@@ -653,54 +642,6 @@ __global__ void __launch_bounds__(kRefineThreads) k_wide_refine(const float4 *le
   refine(nq);
 }
 
-// Any hit: one lane per ray; after a node's box loop the lanes with hit leaf
-// children test those triangles together, whatever slots they are in (testing
-// them inside the child loop ran each slot's test separately with few lanes
-// active), and the first hit ends the ray.
-template <bool BATCHED, bool V8>
-__global__ void __launch_bounds__(kWideThreads, 8)
-    k_trace_wide_any(const WideNode *nodes, const float4 *leaf, const uint32_t *roots, const uint32_t *ray_off,
-                     uint32_t meshes, const float4 *rays, uint64_t nrays, Hit *hits, unsigned long long *counter,
-                     uint32_t *err) {
-  bool active = false, drained = false;
-  uint64_t r = 0;
-  Ray R;
-  uint32_t node = 0, best = kMiss, best_leaf = 0;
-  float bt = 0.0f;
-  __shared__ uint2 s_stack[kWideShared][kWideThreads];
-  uint2 *const sh = &s_stack[0][threadIdx.x];
-  uint2 over[kWideStack - kWideShared], top = make_uint2(0u, 0u);
-  uint32_t warp_mesh = 0;  // a mesh at or below every ray this warp will still take
-  int sp = 0;
-  while (true) {
-    if (wide_take_ray<BATCHED>(active, drained, warp_mesh, r, R, node, roots, ray_off, meshes, rays, nrays,
-                               counter)) {
-      best = kMiss;
-      best_leaf = 0;
-      bt = __fadd_rn(R.tmax, 0.0f);  // never -0 (wide_node_step tests a sign)
-      sp = 0;
-      top.y = 0;
-    }
-    if (!__any_sync(FULL_MASK, active)) {
-      if (drained) break;
-      continue;
-    }
-    if (!active) continue;
-    const WideStep S = wide_node_step<false, V8>(nodes, node, R, bt);
-    uint32_t leaf_hit = S.hm & ~S.imask;
-    while (leaf_hit) {
-      const int c = __ffs(leaf_hit) - 1;
-      leaf_hit &= leaf_hit - 1u;
-      const uint32_t meta = wide_leaf_meta(S, c);
-      if (meta != 0xFF) wide_leaf_test(leaf, S.leaf_base + meta, R, best, best_leaf, bt);
-    }
-    if (best != kMiss || !wide_next<kWideShared>(S, top, sh, over, sp, node, err)) {
-      hits[r] = wide_result(best, best_leaf);
-      active = false;
-    }
-  }
-}
-
 constexpr int kWideFlush = 16;  // queued entries that trigger a flush
 constexpr int kWideSteps = 3;   // node steps between two looks at what else is to be done
 constexpr int kWideQueue = kWideFlush + 32 * kWideSteps;  // a step queues at most 32 entries
@@ -720,6 +661,13 @@ constexpr int kWideQueue = kWideFlush + 32 * kWideSteps;  // a step queues at mo
 // refill.  The closest (t, id) over all tested triangles is the same in any
 // order of tests, so the hits equal the immediate test's; the culling
 // distance only lags.
+// Any hit (ANY) walks on while its tests are queued, and the first entry of a
+// ray with a hit ends it: the key's upper word is then the entry's place in
+// the queue, so the hit is the one that tests run at once would have found
+// (the closest of that entry, ties to the lowest id).  Tests run at once
+// left 16.6 of 32 lanes active: 4.0 M rays on 4.2 M triangles 3.82 -> 3.08 ms
+// with the changes to the step above, 77.5 M rays over 4,096 meshes 25.0 ->
+// 20.3 ms.
 // One entry per lane and step (placing every test by a prefix sum over the
 // lanes in every step took as long as the tests), kWideSteps steps between two
 // looks at flush, refill and finished rays, and 72 registers without spills:
@@ -730,9 +678,9 @@ constexpr int kWideQueue = kWideFlush + 32 * kWideSteps;  // a step queues at mo
 // steps: 4.83 / 4.45 / 4.44 / 4.39 / 4.59 / 4.66 ms; flush at 10 / 16 / 24
 // entries: 4.63 / 4.60 / 4.69 ms; refill at 4 / 6 / 8 idle lanes: 4.30 / 4.30
 // / 4.37 ms, and 25.2 / 24.9 / 24.8 ms on the 4,096 meshes.
-template <bool BATCHED, bool V8>
+template <bool ANY, bool BATCHED, bool V8>
 __global__ void __launch_bounds__(kWideThreads, kWideCtas)
-    k_trace_wide_closest(const WideNode *nodes, const float4 *leaf, const uint32_t *roots, const uint32_t *ray_off,
+    k_trace_wide(const WideNode *nodes, const float4 *leaf, const uint32_t *roots, const uint32_t *ray_off,
                          uint32_t meshes, const float4 *rays, uint64_t nrays, Hit *hits,
                          unsigned long long *counter, uint32_t *err) {
   __shared__ uint2 s_stack[kWideShared][kWideThreads];
@@ -740,6 +688,7 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas)
   __shared__ uint8_t s_list[kWideThreads / 32][256];  // tests of 32 entries: entry | slot << 5
   __shared__ unsigned long long s_best[kWideThreads / 32][32];
   __shared__ uint32_t s_bslot[kWideThreads / 32][32];
+  __shared__ uint32_t s_bid[kWideThreads / 32][ANY ? 32 : 1];  // any hit: the primitive of s_best
   // what only the flush and the final store read stays in shared memory, not
   // in registers
   __shared__ float s_rs[kWideThreads / 32][4][32];  // Sx, Sy, Sz, tmax of each lane's ray
@@ -793,23 +742,35 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas)
         Q.ky = (kk >> 2) & 3;
         Q.kz = kk >> 4;
         unsigned long long key = ~0ull;
+        uint32_t id = 0;
         if (on) {
           const float4 a = __ldg(leaf + 3 * (size_t)slot), bb = __ldg(leaf + 3 * (size_t)slot + 1),
                        c = __ldg(leaf + 3 * (size_t)slot + 2);
           const float v0[3] = {a.x, a.y, a.z}, v1[3] = {bb.x, bb.y, bb.z}, v2[3] = {c.x, c.y, c.z};
           float t;
+          id = __float_as_uint(a.w);
           if (isect_tri(Q, v0, v1, v2, t)) {
-            key = ((unsigned long long)t_order(t) << 32) | __float_as_uint(a.w);
+            key = ANY ? ((unsigned long long)(b + (int)(code & 31u)) << 32) | t_order(t)
+                      : ((unsigned long long)t_order(t) << 32) | id;
             atomicMin(&sbest[o], key);
           }
         }
         __syncwarp();
-        if (key != ~0ull && sbest[o] == key) sbslot[o] = slot;  // one winner per owner
+        bool won = key != ~0ull && sbest[o] == key;
+        if constexpr (ANY) {  // the same entry and distance: the lowest id
+          if (won) s_bid[wq][o] = kMiss;
+          __syncwarp();
+          if (won) atomicMin(&s_bid[wq][o], id);
+          __syncwarp();
+          won = won && s_bid[wq][o] == id;
+        }
+        if (won) sbslot[o] = slot;  // one winner per owner
         __syncwarp();
       }
     }
     if (pending) {
-      bt = t_from_order((uint32_t)(sbest[lane] >> 32));
+      if (!ANY) bt = t_from_order((uint32_t)(sbest[lane] >> 32));
+      else if (sbest[lane] != ~0ull) walking = false;
       pending = false;
     }
     nq = 0;
@@ -822,7 +783,7 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas)
       sp = 0;
       top.y = 0;
       walking = true;
-      sbest[lane] = ((unsigned long long)t_order(R.tmax) << 32) | kMiss;
+      sbest[lane] = ANY ? ~0ull : ((unsigned long long)t_order(R.tmax) << 32) | kMiss;
       s_rs[wq][0][lane] = R.Sx;
       s_rs[wq][1][lane] = R.Sy;
       s_rs[wq][2][lane] = R.Sz;
@@ -838,7 +799,7 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas)
     for (int step = 0; step < kWideSteps; ++step) {
       uint32_t lh = 0, lbase = 0;
       if (walking) {
-        const WideStep S = wide_node_step<true, V8>(nodes, node, R, bt);
+        const WideStep S = wide_node_step<!ANY, V8>(nodes, node, R, bt);
         lbase = S.leaf_base;
         lh = S.hm & ~S.imask;
         // an empty slot (meta 0xFF; only an infinite scale lets one pass the
@@ -857,7 +818,8 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas)
     const unsigned running = __ballot_sync(FULL_MASK, walking);
     if (nq >= kWideFlush || (waiting && (!running || 32 - __popc(running) >= kWideRefill))) flush();
     if (active && !walking && !pending) {
-      hits[s_rid[wq][lane]] = wide_result((uint32_t)sbest[lane], sbslot[lane]);
+      const uint32_t prim = !ANY ? (uint32_t)sbest[lane] : (sbest[lane] != ~0ull ? s_bid[wq][lane] : kMiss);
+      hits[s_rid[wq][lane]] = wide_result(prim, sbslot[lane]);
       active = false;
     }
   }
@@ -949,8 +911,7 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuWideTrace(const gprtcuWideBvh *bvh, con
   ScratchHeader *hdr = (ScratchHeader *)scratch;
   unsigned long long *counter = reinterpret_cast<unsigned long long *>(&hdr->ticket[0]);
   GPRTCU_TRY(cudaMemsetAsync(scratch, 0, sizeof(ScratchHeader), stream));
-  // any hit: 64 registers, 8 CTAs of 128 threads per SM; closest hit: 72, 7
-  const int blocks = gprtcu_num_sms() * (anyHit ? 8 : kWideCtas);
+  const int blocks = gprtcu_num_sms() * kWideCtas;
   const uint64_t need = (numRays + kWideThreads - 1) / kWideThreads;
   const int grid = (int)(need < (uint64_t)blocks ? need : blocks);
   auto launch = [&](auto kernel) {
@@ -960,8 +921,8 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuWideTrace(const gprtcuWideBvh *bvh, con
   };
   auto pick = [&](auto v8) {
     constexpr bool V = decltype(v8)::value;
-    if (numMeshes > 1) anyHit ? launch(k_trace_wide_any<true, V>) : launch(k_trace_wide_closest<true, V>);
-    else anyHit ? launch(k_trace_wide_any<false, V>) : launch(k_trace_wide_closest<false, V>);
+    if (numMeshes > 1) anyHit ? launch(k_trace_wide<true, true, V>) : launch(k_trace_wide<false, true, V>);
+    else anyHit ? launch(k_trace_wide<true, false, V>) : launch(k_trace_wide<false, false, V>);
   };
   if (((uintptr_t)bvh->nodes & 31) == 0) pick(std::true_type());
   else pick(std::false_type());
