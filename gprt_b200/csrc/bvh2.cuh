@@ -131,6 +131,152 @@ __device__ __forceinline__ bool walk_next(Walk &W, float2 *sh, float2 *over, boo
   return ok;
 }
 
+// ---------------------------------------------------------------------------
+// few rays
+// ---------------------------------------------------------------------------
+// Closest hit of few rays: a warp takes up to kPoolRays rays and all its lanes
+// work on them.  With a lane per ray the time of a small call is the chain of
+// its longest ray's node visits, a load and some 250 cycles of arithmetic each
+// (4,099 rays on 1,501 triangles: 66 us), while most lanes have no ray.  Here
+// the nodes still to visit of all the warp's rays are one stack in shared
+// memory, (node, ray, entry distance); every step each lane takes one of its
+// top 32 entries, tests both children and pushes those to enter, the nearer
+// ones last; leaf children go to a second list whose primitive tests run 32 at
+// a time.  A ray's chain is then its depth plus its share of the warp's visits
+// divided by 32.  Whole calls, lane per ray / pooled: 4,099 rays on 1,501
+// triangles 80 / 30 us, on 262,144 triangles 210 / 38 us; 40,001 rays there
+// 348 / 156 us, 113,001 403 / 362 us; from there the lane per ray is faster
+// (200,001: 558 / 627 us; 1,048,576: 1.94 / 2.9 ms), since nearer nodes are not
+// strictly first and every step reads its ray from shared memory.  The closest
+// (t, id) is the same in any order.  Where boxes overlap so much that nearly
+// every child is entered, the stack grows to the lanes times the tree's depth;
+// from kPoolWide entries on, fewer lanes go on the fuller it is (an eighth of
+// what is left), in the end one, whose walk needs no more than the tree's
+// depth on top.
+constexpr int kPoolRays = 16;
+constexpr int kPoolStack = 456;              // entries; a step pops up to 32 and pushes at most 64
+constexpr int kPoolWide = 128;               // up to here all lanes go on
+static_assert(kPoolStack - 64 - kPoolWide >= 8 * 32, "all lanes at the line");
+constexpr int kPoolLeaves = 96;              // a step queues at most 64
+constexpr int kPoolThreads = 64;
+constexpr int kPoolWarps = kPoolThreads / 32;
+constexpr int kPoolCtas = 12;
+constexpr int kPoolRounds = 2;  // chunks of kPoolRays per warp up to which rays are few
+
+struct PoolShared {
+  uint2 stack[kPoolStack];  // node, entry distance
+  float4 ray[kPoolRays][2];  // {-origin, tmin}, {1 / direction, tmax}
+  unsigned long long best[kPoolRays];  // closest (t, id)
+  uint32_t base[kPoolRays][2];         // first leaf slot and node of the ray's mesh
+  uint32_t leaf[kPoolLeaves];
+  uint8_t sray[kPoolStack], lray[kPoolLeaves];
+};
+__device__ __forceinline__ void pool_ray(PoolShared &S, int ray, const Ray &R, uint32_t base_leaf,
+                                         uint32_t base_node) {
+  S.ray[ray][0] = make_float4(-R.ox, -R.oy, -R.oz, R.tmin);
+  S.ray[ray][1] = make_float4(R.ix, R.iy, R.iz, R.tmax);
+  S.best[ray] = ((unsigned long long)t_order(R.tmax) << 32) | kMiss;
+  S.base[ray][0] = base_leaf;
+  S.base[ray][1] = base_node;
+}
+// All 32 lanes call; lane i's ray (set by pool_ray) starts at its mesh's root
+// (root), or has the single leaf of a mesh without inner nodes to test (one).
+// PRIMS: test(slot, ray, {-o, tmin}, {1/d, tmax}, aux) gives the (t, id) key
+// of a hit or ~0; won(ray, slot, aux) is called for a hit that became the
+// ray's best.  False when the stack was too small for the tree.
+template <bool BATCHED, bool V8, class PRIMS>
+__device__ __forceinline__ bool pool_walk(PoolShared &S, const Bvh2Node *bvh, bool root, bool one,
+                                          const PRIMS &prims) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt = (1u << lane) - 1u;
+  const float kNone = __int_as_float(0x7fffffff);
+  int ns = 0, nl = 0;  // stack entries, queued leaves: the same on every lane
+  auto push = [&](bool want, int node, float tn, int ray) {
+    const unsigned m = __ballot_sync(FULL_MASK, want);
+    if (want) {
+      const int k = ns + __popc(m & lt);
+      S.stack[k] = make_uint2((uint32_t)node, __float_as_uint(tn));
+      S.sray[k] = (uint8_t)ray;
+    }
+    ns += __popc(m);
+  };
+  auto queue = [&](bool want, uint32_t slot, int ray) {
+    const unsigned m = __ballot_sync(FULL_MASK, want);
+    if (want) {
+      const int k = nl + __popc(m & lt);
+      S.leaf[k] = slot;
+      S.lray[k] = (uint8_t)ray;
+    }
+    nl += __popc(m);
+  };
+  auto flush = [&]() {  // the last up to 32 queued primitive tests
+    const int k = nl < 32 ? nl : 32;
+    nl -= k;
+    __syncwarp();
+    unsigned long long key = ~0ull;
+    uint32_t slot = 0;
+    int ray = 0;
+    float aux = 0.0f;
+    if (lane < k) {
+      slot = S.leaf[nl + lane];
+      ray = S.lray[nl + lane];
+      key = prims.test(slot, ray, S.ray[ray][0], S.ray[ray][1], aux);
+      if (key != ~0ull) atomicMin(&S.best[ray], key);
+    }
+    __syncwarp();
+    if (key != ~0ull && S.best[ray] == key) prims.won(ray, slot, aux);  // one winner per ray
+    __syncwarp();
+  };
+  __syncwarp();
+  push(root, root ? (int)S.base[lane][1] : 0, 0.0f, lane);
+  queue(one, one ? S.base[lane][0] : 0u, lane);
+  while (true) {
+    __syncwarp();
+    if (nl >= 32 || (ns == 0 && nl > 0)) flush();
+    if (ns == 0) {
+      if (nl == 0) break;
+      continue;
+    }
+    const int k = ns <= kPoolWide ? min(ns, 32) : max(min((kPoolStack - 64 - ns) >> 3, 32), 1);
+    if (ns + k > kPoolStack) return false;
+    ns -= k;
+    int ray = 0, r0 = 0, r1 = 0;
+    float t0 = kNone, t1 = kNone;
+    bool leaf0 = false, leaf1 = false;
+    if (lane < k) {
+      const uint2 e = S.stack[ns + lane];
+      ray = S.sray[ns + lane];
+      const float bt = t_from_order((uint32_t)(S.best[ray] >> 32));
+      if (__uint_as_float(e.y) <= bt) {
+        const Bvh2Node *nd = bvh + e.x;
+        const ChildPairs c0 = load_child<V8>(&nd->c[0]), c1 = load_child<V8>(&nd->c[1]);
+        const float4 o = S.ray[ray][0], i = S.ray[ray][1];
+        const RayPairs P{pk2(o.x, o.y), pk2(o.z, o.z), pk2(i.x, i.y), pk2(i.z, i.z), o.w};
+        t0 = child_entry(c0, P, bt);
+        t1 = child_entry(c1, P, bt);
+        r0 = c0.ref;
+        r1 = c1.ref;
+        leaf0 = r0 < 0 && t0 == t0;
+        leaf1 = r1 < 0 && t1 == t1;
+      }
+    }
+    __syncwarp();  // the entries are taken before others go over them
+    const bool in0 = r0 >= 0 && t0 == t0, in1 = r1 >= 0 && t1 == t1;
+    const bool near0 = in0 && !(in1 && t1 < t0);
+    const int bn = BATCHED ? (int)S.base[ray][1] : 0;
+    const uint32_t bl = BATCHED ? S.base[ray][0] : 0u;
+    push(in0 && in1, bn + (near0 ? r1 : r0), near0 ? t1 : t0, ray);
+    push(in0 || in1, bn + (near0 ? r0 : r1), near0 ? t0 : t1, ray);
+    if (__any_sync(FULL_MASK, leaf0 || leaf1)) {
+      while (nl > kPoolLeaves - 64) flush();
+      queue(leaf0, bl + (uint32_t)~r0, ray);
+      queue(leaf1, bl + (uint32_t)~r1, ray);
+    }
+  }
+  __syncwarp();
+  return true;
+}
+
 // Idle lanes take new rays from the global counter once `refill` of the
 // warp's `lanes` are idle (or all are).  Returns true on the lanes that took
 // one, its index in r.  All 32 lanes call.
@@ -154,18 +300,32 @@ __device__ __forceinline__ bool warp_take(bool active, bool &drained, int lanes,
 
 // Grid of a persistent ray kernel (`ctas` CTAs of `warps` warps fit on an SM)
 // and the rays a warp holds at a time: all 32 lanes once there are rays for
-// every warp that fits on the GPU; fewer rays are spread over the warps
+// kSpreadWarps warps per SM; fewer rays are spread over that many warps
 // instead, at least four to each (a warp's time is that of its longest ray,
 // and lanes without a ray still run queued primitive tests).  4,099 rays on
-// 1,501 triangles at 32 / 16 / 8 / 4 / 2 / 1 rays per warp: 102 / 85 / 81 /
-// 78 / 78 / 93 us.
+// 1,501 triangles at 32 / 16 / 8 / 4 / 2 / 1 rays per warp: 102 / 85 / 81 / 78
+// / 78 / 93 us.  Spread over every warp that fits (32 per SM) the warps' own
+// instructions add up: 18,001 rays on 262,144 triangles, any hit, 335 us
+// against 272 us.
+constexpr int kSpreadWarps = 8;
 struct RayGrid {
   int ctas, lanes;
 };
 static inline RayGrid ray_grid(uint64_t nrays, int ctas, int warps) {
   const uint64_t fit = (uint64_t)gprtcu_num_sms() * ctas;
-  const uint64_t share = (nrays + fit * warps - 1) / (fit * warps);
+  const uint64_t spread = (uint64_t)gprtcu_num_sms() * kSpreadWarps;
+  const uint64_t share = (nrays + spread - 1) / spread;
   const int lanes = share >= 32 ? 32 : (share < 4 ? 4 : (int)share);
   const uint64_t need = (nrays + (uint64_t)lanes * warps - 1) / ((uint64_t)lanes * warps);
+  return RayGrid{(int)(need < fit ? need : fit), lanes};
+}
+// Grid of a pool kernel and the rays a warp takes at a time (two at least); 0
+// rays when there are too many for it.
+static inline RayGrid pool_grid(uint64_t nrays) {
+  const uint64_t fit = (uint64_t)gprtcu_num_sms() * gprtcu::kPoolCtas, warps = fit * gprtcu::kPoolWarps;
+  if (nrays > warps * gprtcu::kPoolRays * gprtcu::kPoolRounds) return RayGrid{0, 0};
+  const uint64_t share = (nrays + warps - 1) / warps;
+  const int lanes = share > gprtcu::kPoolRays ? gprtcu::kPoolRays : (share < 2 ? 2 : (int)share);
+  const uint64_t need = (nrays + (uint64_t)lanes * gprtcu::kPoolWarps - 1) / ((uint64_t)lanes * gprtcu::kPoolWarps);
   return RayGrid{(int)(need < fit ? need : fit), lanes};
 }

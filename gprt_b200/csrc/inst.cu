@@ -136,7 +136,6 @@ constexpr int kInstWarps = kInstThreads / 32;
 constexpr int kInstShared = 10;  // stack entries in shared memory
 constexpr int kInstDepth = 128;  // 62 levels of each tree
 constexpr int kInstRefill = 4;
-constexpr int kInstEnter = 8;
 constexpr int kInstSteps = 6;
 constexpr int kInstFlush = 12;
 constexpr int kInstQueue = 96;  // a step queues at most 64
@@ -175,23 +174,23 @@ __device__ __forceinline__ void inst_refine(const InstArgs &A, const InstRefineQ
 }
 
 // One lane per ray from a global counter.  A lane walks the top level with
-// its world ray; an instance it reaches waits until kInstEnter lanes of the
-// warp want to enter one (or no lane can do anything else), then these map
-// their rays into object space together -- two divisions, four reciprocals
-// and twelve loads that a lane alone would keep the warp waiting for -- and
-// walk that mesh on the same stack, above a mark that leads back to the top
-// level.  Closest hit queues its triangle tests per warp and runs them with all
-// lanes (as the one-level traversal does); the queue is emptied before a lane
-// with tests in it enters another instance, so the tests of a lane all belong
-// to the instance it entered last, whose object-space ray is in shared memory.
+// its world ray; the lanes that reach an instance within the same few steps
+// map their rays into object space together and walk that mesh on the same
+// stack, above a mark that leads back to the top level.  Closest hit queues its
+// triangle tests per warp and runs them with all lanes (as the one-level
+// traversal does); the queue is emptied before a lane with tests in it enters
+// another instance, so the tests of a lane all belong to the instance it
+// entered last, whose object-space ray is in shared memory.
 // With entries, node steps and tests of single lanes each taking the whole
 // warp's time, 7.6 of 32 lanes were active; now 19 are, and the L1 data pipe
 // (76 % busy, see load_child) and load latency bound it.  4.2 M rays over
-// 16,384 instances: 18.0 -> 10.8 ms.  Entering at 1 / 4 / 6 / 8 / 12 waiting
-// lanes: 12.8 / 12.3 / 10.8 / 10.8 / 11.1 ms (the first two before the CTAs
-// per SM went from 6 to 8, 12.1 -> 10.8 ms); 2 / 4 / 6 / 8 node steps between
-// two looks at entries, flush and refill: 12.5 / 12.1 / 11.2 / 12.0 ms then.
-// 10 stack entries in shared memory against 8 and 6: 10.8 / 11.2 / 11.5 ms.
+// 16,384 instances: 18.0 -> 10.9 ms; 200,001 rays: 1.39 -> 1.01 ms.  Letting
+// entering lanes wait for 2 / 4 / 8 of them: 10.9 / 10.9 / 10.9 ms and 1.04 /
+// 1.14 / 1.31 ms (and 0.33 / 0.38 / 0.40 / 0.45 ms for 1 / 2 / 4 / 8 on 200,001
+// rays over 1,001 instances, 0.37 before).  8 CTAs per SM instead of 6: 12.1 ->
+// 10.8 ms; 2 / 4 / 6 / 8 node steps between two looks at entries, flush and
+// refill: 12.5 / 12.1 / 11.2 / 12.0 ms then.  10 stack entries in shared memory
+// against 8 and 6: 10.8 / 11.2 / 11.5 ms.
 template <bool ANY, bool V8>
 __global__ void __launch_bounds__(kInstThreads, kInstCtas) k_trace_inst(const InstArgs A) {
   __shared__ float2 s_stack[kInstShared][kInstThreads];
@@ -376,9 +375,8 @@ __global__ void __launch_bounds__(kInstThreads, kInstCtas) k_trace_inst(const In
       }
     }
     // ---- instances: enter them together
-    const unsigned walking = __ballot_sync(FULL_MASK, W.node >= 0);
     const unsigned entering = __ballot_sync(FULL_MASK, W.node < 0 && W.node > kWalkLeave);
-    if (entering && (!walking || __popc(entering) >= kInstEnter)) {
+    if (entering) {
       const bool enter = W.node < 0 && W.node > kWalkLeave;
       if (!ANY && __any_sync(FULL_MASK, enter && pending)) flush();
       if (!ANY && nq > kInstQueue - 32) flush();

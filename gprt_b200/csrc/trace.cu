@@ -393,6 +393,96 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_closest(con
   refine_queued(A, rq, 0, nrq);
 }
 
+// The triangle tests of pool_walk (few rays) and what they need of a ray
+// besides its origin, reciprocal direction, tmin and tmax.
+struct PoolTriangles {
+  const float4 *leaf;
+  float4 *shear;  // per ray {Sx, Sy, Sz, kx | ky << 2 | kz << 4}
+  uint32_t *slot;  // leaf slot of each ray's best hit
+  __device__ __forceinline__ unsigned long long test(uint32_t s, int ray, const float4 &o, const float4 &i,
+                                                     float &) const {
+    const float4 q = shear[ray];
+    Ray Q;
+    Q.ox = -o.x;
+    Q.oy = -o.y;
+    Q.oz = -o.z;
+    Q.tmin = o.w;
+    Q.tmax = i.w;
+    Q.Sx = q.x;
+    Q.Sy = q.y;
+    Q.Sz = q.z;
+    const int k = __float_as_int(q.w);
+    Q.kx = k & 3;
+    Q.ky = (k >> 2) & 3;
+    Q.kz = k >> 4;
+    const float4 a = __ldg(leaf + 3 * (size_t)s), b = __ldg(leaf + 3 * (size_t)s + 1),
+                 c = __ldg(leaf + 3 * (size_t)s + 2);
+    const float v0[3] = {a.x, a.y, a.z}, v1[3] = {b.x, b.y, b.z}, v2[3] = {c.x, c.y, c.z};
+    float t;
+    if (!isect_tri(Q, v0, v1, v2, t)) return ~0ull;
+    return ((unsigned long long)t_order(t) << 32) | __float_as_uint(a.w);
+  }
+  __device__ __forceinline__ void won(int ray, uint32_t s, float) const { slot[ray] = s; }
+};
+
+template <bool BATCHED, bool V8>
+__global__ void __launch_bounds__(kPoolThreads, kPoolCtas) k_trace_pool(const TraceArgs A) {
+  __shared__ PoolShared s_pool[kPoolWarps];
+  __shared__ float4 s_shear[kPoolWarps][kPoolRays];
+  __shared__ uint32_t s_bslot[kPoolWarps][kPoolRays];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  PoolShared &S = s_pool[w];
+  const PoolTriangles tris{A.leaf, s_shear[w], s_bslot[w]};
+  while (true) {
+    unsigned long long first = 0;
+    if (lane == 0) first = atomicAdd(A.counter, (unsigned long long)A.lanes);
+    first = __shfl_sync(FULL_MASK, first, 0);
+    if (first >= A.nrays) break;
+    const uint64_t r = first + lane;
+    const bool mine = lane < A.lanes && r < A.nrays;
+    bool one = false, root = false;
+    uint32_t base_leaf = 0, base_node = 0;
+    if (mine) {
+      Ray R;
+      ray_setup(__ldg(A.rays + 2 * r), __ldg(A.rays + 2 * r + 1), R);
+      uint32_t n = A.n;
+      if (BATCHED) {
+        const uint32_t m = mesh_of_ray(A.tm, r);
+        base_leaf = __ldg(A.tm.tri_off + m);
+        n = __ldg(A.tm.tri_off + m + 1) - base_leaf;
+        base_node = base_leaf - m;
+      }
+      pool_ray(S, lane, R, base_leaf, base_node);
+      s_shear[w][lane] = make_float4(R.Sx, R.Sy, R.Sz, __int_as_float(R.kx | (R.ky << 2) | (R.kz << 4)));
+      root = n > 1;
+      one = n == 1 && single_leaf_box(A.leaf, base_leaf, R);
+    }
+    if (!pool_walk<BATCHED, V8>(S, A.bvh, root, one, tris)) {
+      if (lane == 0) atomicCAS(A.err, 0u, 5u);  // traversal stack overflow
+      break;
+    }
+    if (mine) {
+      const unsigned long long key = S.best[lane];
+      Hit h;
+      h.prim = (uint32_t)key;
+      h.t = __int_as_float(0x7f800000);
+      if (h.prim != kMiss) {
+        const uint32_t slot = s_bslot[w][lane];
+        const float4 o = __ldg(A.rays + 2 * r), d = __ldg(A.rays + 2 * r + 1);
+        Ray R;
+        R.ox = o.x; R.oy = o.y; R.oz = o.z;
+        R.dx = d.x; R.dy = d.y; R.dz = d.z;
+        const float4 a = __ldg(A.leaf + 3 * (size_t)slot), b = __ldg(A.leaf + 3 * (size_t)slot + 1),
+                     c = __ldg(A.leaf + 3 * (size_t)slot + 2);
+        const float v0[3] = {a.x, a.y, a.z}, v1[3] = {b.x, b.y, b.z}, v2[3] = {c.x, c.y, c.z};
+        h.t = refine_t(R, v0, v1, v2);
+      }
+      A.hits[r] = h;
+    }
+    __syncwarp();
+  }
+}
+
 }  // namespace gprtcu
 
 using namespace gprtcu;
@@ -426,18 +516,26 @@ gprtcuStatus trace_launch(const gprtcuLbvh *bvh, const uint32_t *tri_off, const 
   a.counter = counter;
   a.err = &hdr->status;
   const bool v8 = ((uintptr_t)bvh->bvh2 & 31) == 0;
-#define GPRTCU_TRACE(K)                                                             \
-  do {                                                                              \
-    if (meshes > 1) {                                                               \
-      if (v8) K<true, true><<<g.ctas, kTraceThreads, 0, stream>>>(a);               \
-      else K<true, false><<<g.ctas, kTraceThreads, 0, stream>>>(a);                   \
-    } else {                                                                        \
-      if (v8) K<false, true><<<g.ctas, kTraceThreads, 0, stream>>>(a);                \
-      else K<false, false><<<g.ctas, kTraceThreads, 0, stream>>>(a);                  \
-    }                                                                               \
+#define GPRTCU_LAUNCH(K, CTAS, THREADS)                                 \
+  do {                                                                  \
+    if (meshes > 1) {                                                   \
+      if (v8) K<true, true><<<CTAS, THREADS, 0, stream>>>(a);           \
+      else K<true, false><<<CTAS, THREADS, 0, stream>>>(a);             \
+    } else {                                                            \
+      if (v8) K<false, true><<<CTAS, THREADS, 0, stream>>>(a);          \
+      else K<false, false><<<CTAS, THREADS, 0, stream>>>(a);            \
+    }                                                                   \
   } while (0)
-  if (any) GPRTCU_TRACE(k_trace_any);
-  else GPRTCU_TRACE(k_trace_closest);
+#define GPRTCU_TRACE(K) GPRTCU_LAUNCH(K, g.ctas, kTraceThreads)
+  if (any) {
+    GPRTCU_TRACE(k_trace_any);
+  } else if (const RayGrid few = pool_grid(nrays); few.lanes) {
+    a.lanes = few.lanes;
+    GPRTCU_LAUNCH(k_trace_pool, few.ctas, kPoolThreads);
+  } else {
+    GPRTCU_TRACE(k_trace_closest);
+  }
+#undef GPRTCU_LAUNCH
 #undef GPRTCU_TRACE
   GPRTCU_TRY(cudaGetLastError());
   return GPRTCU_OK;

@@ -407,6 +407,76 @@ __global__ void __launch_bounds__(kUserThreads, kUserCtas) k_trace_user(const Us
   }
 }
 
+// The primitive tests of pool_walk (few rays): the ray's direction, and u of
+// its best hit, per ray.
+template <typename PRIMS> struct PoolPrims {
+  const UserArgs<PRIMS> &A;
+  float4 *dir;
+  float *u;
+  __device__ __forceinline__ unsigned long long test(uint32_t s, int ray, const float4 &o, const float4 &i,
+                                                     float &hu) const {
+    const float4 d = dir[ray];
+    Ray Q;
+    Q.ox = -o.x;
+    Q.oy = -o.y;
+    Q.oz = -o.z;
+    Q.tmin = o.w;
+    Q.dx = d.x;
+    Q.dy = d.y;
+    Q.dz = d.z;
+    Q.tmax = i.w;
+    const uint32_t id = __ldg(A.ids + s);
+    float t;
+    if (!A.prims.hit(Q, id, A.exit_test, t, hu)) return ~0ull;
+    return ((unsigned long long)t_order(t) << 32) | id;
+  }
+  __device__ __forceinline__ void won(int ray, uint32_t, float hu) const { u[ray] = hu; }
+};
+
+template <typename PRIMS, bool V8>
+__global__ void __launch_bounds__(kPoolThreads, kPoolCtas) k_user_pool(const UserArgs<PRIMS> A) {
+  __shared__ PoolShared s_pool[kPoolWarps];
+  __shared__ float4 s_dir[kPoolWarps][kPoolRays];
+  __shared__ float s_u[kPoolWarps][kPoolRays];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  PoolShared &S = s_pool[w];
+  const PoolPrims<PRIMS> prims{A, s_dir[w], s_u[w]};
+  while (true) {
+    unsigned long long first = 0;
+    if (lane == 0) first = atomicAdd(A.counter, (unsigned long long)A.lanes);
+    first = __shfl_sync(FULL_MASK, first, 0);
+    if (first >= A.nrays) break;
+    const uint64_t r = first + lane;
+    const bool mine = lane < A.lanes && r < A.nrays;
+    bool one = false;
+    if (mine) {
+      Ray R;
+      ray_setup(__ldg(A.rays + 2 * r), __ldg(A.rays + 2 * r + 1), R);
+      pool_ray(S, lane, R, 0u, 0u);
+      s_dir[w][lane] = make_float4(R.dx, R.dy, R.dz, 0.0f);
+      if (A.n == 1) {
+        float tn;
+        one = ray_box(R, A.root_box[0], A.root_box[1], A.root_box[2], A.root_box[3], A.root_box[4], A.root_box[5],
+                      R.tmax, tn);
+      }
+    }
+    if (!pool_walk<false, V8>(S, A.bvh, mine && A.n > 1, one, prims)) {
+      if (lane == 0) atomicCAS(A.err, 0u, 5u);  // traversal stack overflow
+      break;
+    }
+    if (mine) {
+      const unsigned long long key = S.best[lane];
+      const bool hit = (uint32_t)key != kMiss;
+      Hit h;
+      h.prim = (uint32_t)key;
+      h.t = hit ? t_from_order((uint32_t)(key >> 32)) : __int_as_float(0x7f800000);
+      A.hits[r] = h;
+      if (A.hit_u) A.hit_u[r] = hit ? s_u[w][lane] : 0.0f;
+    }
+    __syncwarp();
+  }
+}
+
 }  // namespace gprtcu
 
 using namespace gprtcu;
@@ -436,7 +506,11 @@ gprtcuStatus trace_user(const gprtcuLbvh *bvh, PRIMS prims, const float *rays, u
                     (const float4 *)rays, nrays, g.lanes, (Hit *)hits, u, counter, &hdr->status};
   auto launch = [&](auto kernel) { kernel<<<g.ctas, kUserThreads, 0, stream>>>(a); };
   const bool v8 = ((uintptr_t)bvh->bvh2 & 31) == 0;
-  if (any) v8 ? launch(k_trace_user<PRIMS, true, true>) : launch(k_trace_user<PRIMS, true, false>);
+  if (const RayGrid few = pool_grid(nrays); !any && few.lanes) {
+    a.lanes = few.lanes;
+    if (v8) k_user_pool<PRIMS, true><<<few.ctas, kPoolThreads, 0, stream>>>(a);
+    else k_user_pool<PRIMS, false><<<few.ctas, kPoolThreads, 0, stream>>>(a);
+  } else if (any) v8 ? launch(k_trace_user<PRIMS, true, true>) : launch(k_trace_user<PRIMS, true, false>);
   else v8 ? launch(k_trace_user<PRIMS, false, true>) : launch(k_trace_user<PRIMS, false, false>);
   GPRTCU_TRY(cudaGetLastError());
   return GPRTCU_OK;

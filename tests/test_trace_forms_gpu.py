@@ -50,6 +50,19 @@ def test_trace_forms(cuda, n, m, shift):
     assert np.array_equal(anyh["prim"] != 0xFFFFFFFF, exp["prim"] != 0xFFFFFFFF)
 
 
+@pytest.mark.parametrize("n,m", [(40, 700), (5000, 300), (60000, 64)])
+def test_trace_overlapping(cuda, n, m):
+    """Triangles as large as the scene: nearly every box is entered, and the
+    shared stack of the few-ray form fills up."""
+    import torch
+    from gprt_b200 import api
+    pos, tri = scenes.soup(n, seed=3, sigma=1.0)
+    rays = scenes.rays(m, seed=4)
+    rays[::3, 7] = 0.9
+    b = api.lbvh_build_triangles(torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda())
+    assert _same(api.hits_numpy(api.trace(b, torch.from_numpy(rays).cuda())), _expect(pos, tri, rays))
+
+
 @pytest.mark.parametrize("shift", [0, 16])
 def test_batch_trace_forms(cuda, shift):
     import torch
