@@ -169,6 +169,47 @@ def test_prims_forms(cuda, m):
             assert np.array_equal(h0["prim"], e["prim"])
 
 
+def _odd_rays(m, seed, share):
+    """Rays with some components infinite, NaN, zero or huge."""
+    rng = np.random.default_rng(seed)
+    rays = scenes.rays(m, seed=seed)
+    odd = np.float32([np.nan, np.inf, -np.inf, 0.0, -0.0, -1.0, 1e30, -1e30, 1e-40, 3.4e38])
+    rays = np.where(rng.random((m, 8)) < share, odd[rng.integers(0, odd.size, (m, 8))], rays).astype(np.float32)
+    rays[::97, 4:7] = 0.0  # no direction
+    return rays
+
+
+@pytest.mark.parametrize("n", [1, 300])
+def test_prims_odd_rays(cuda, n):
+    """Rays whose primitive tests can give a distance that is no number: such
+    a hit counts if it is the ray's first.  One primitive: as the oracle says;
+    more: the same however many rays the call has."""
+    import torch
+    from gprt_b200 import api
+    few, many = 4099, 151553
+    rng = np.random.default_rng(n)
+    v = np.concatenate([rng.random((n + 1, 3)), rng.uniform(0.1, 0.3, (n + 1, 1))], 1).astype(np.float32)
+    idx = np.stack([np.arange(n), np.arange(n) + 1], 1).astype(np.uint32)
+    vt, it = torch.from_numpy(v).cuda(), torch.from_numpy(idx.view(np.int32)).cuda()
+    rays_h = _odd_rays(many, n, 0.05)
+    rays = torch.from_numpy(rays_h).cuda()
+    for kind in (0, 1):
+        b = api.lbvh_build_boxes(api.sphere_bounds(vt[:n]) if kind == 0 else api.lss_bounds(vt, it))
+        run = (lambda r, **k: api.hits_numpy(api.trace_spheres(b, vt[:n], r, **k))) if kind == 0 else \
+            (lambda r, **k: api.hits_numpy(api.trace_lss(b, vt, it, r, **k)))
+        u = torch.zeros(many, device="cuda"), torch.zeros(few, device="cuda")
+        full, part, anyh = run(rays, u=u[0]), run(rays[:few].contiguous(), u=u[1]), run(rays, anyhit=True)
+        assert np.isnan(full["t"]).sum() > 50
+        assert np.array_equal(full[:few].view(np.uint32), part.view(np.uint32))
+        assert torch.equal(u[0][:few].view(torch.int32), u[1].view(torch.int32))
+        assert np.array_equal(full["prim"] == 0xFFFFFFFF, anyh["prim"] == 0xFFFFFFFF)
+        if n == 1:
+            e = oracle.trace_user_brute(kind, v[:n] if kind == 0 else v, rays_h, *(() if kind == 0 else (idx,)))
+            hit = full["prim"] == 0  # the box test may drop a ray that the primitive test alone would not
+            assert np.all(e["prim"][hit] == 0)
+            assert np.array_equal(np.isnan(full["t"][hit]), np.isnan(e["t"][hit]))
+
+
 @pytest.mark.parametrize("stride", [32, 36, 48])
 @pytest.mark.parametrize("shift", [0, 16])
 def test_solid_forms(cuda, stride, shift):
