@@ -7,6 +7,7 @@
 // child is entered when its entry distance does not exceed the best hit
 // (equal distance still enters, so a tie can be won by a lower primitive id).
 // Leaf triangles are stored in leaf order.
+#include <type_traits>
 #include "bvh2.cuh"
 #include "common.cuh"
 #include "lbvh.cuh"
@@ -122,11 +123,24 @@ __device__ __forceinline__ void finish_rays(const TraceArgs &A, RefineQueue &q, 
 // one; base_leaf and base_node are the first leaf slot and node of the ray's
 // mesh and n its triangles.
 constexpr int kTraceRefill = 8;
+// One mesh whose nodes and leaves (112 bytes a triangle) pass some 560 MB: a
+// node that is not in L2 costs so much more from there on that rays which
+// start together are worth more than full lanes, since they meet in the upper
+// nodes; most of the lanes, then all, have to be idle first.  Rays per call
+// as many as triangles, refill at 8 / 24 / 32: 4.2 M 5.7 / 6.8 / 10.2 ms, 6.0
+// M 13.5 / 11.6 / 15.6, 8.4 M 25.5 / 21.2 / 23.2; 4.2 M rays on 16.8 M
+// triangles 66 / 56 / 52 ms, on 33.6 M 18.5 / 15.8 / 15.5 (any hit alike).
+// The meshes of a batch are small, and a warp's rays are of one or two.
+// (An argument instead of a template parameter cost 3 %.)
+static inline int trace_refill(uint32_t n, uint32_t meshes) {
+  if (meshes > 1 || n <= 5000000u) return kTraceRefill;
+  return n <= 12000000u ? 24 : 32;
+}
 
-template <bool BATCHED>
+template <bool BATCHED, int REFILL>
 __device__ __forceinline__ bool take_rays(const TraceArgs &A, bool active, bool &drained, uint64_t &r, Ray &R,
                                           uint32_t &n, uint32_t &base_leaf, uint32_t &base_node) {
-  if (!warp_take(active, drained, A.lanes, kTraceRefill, A.nrays, A.counter, r)) return false;
+  if (!warp_take(active, drained, A.lanes, REFILL, A.nrays, A.counter, r)) return false;
   ray_setup(__ldg(A.rays + 2 * r), __ldg(A.rays + 2 * r + 1), R);
   n = A.n;
   base_leaf = base_node = 0;
@@ -142,7 +156,7 @@ __device__ __forceinline__ bool take_rays(const TraceArgs &A, bool active, bool 
 
 // Any hit: a lane tests the leaf triangles it meets at once, and the first
 // step with a hit ends its ray.
-template <bool BATCHED, bool V8>
+template <bool BATCHED, bool V8, int REFILL>
 __global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_any(const TraceArgs A) {
   __shared__ float2 s_stack[kStackShared][kTraceThreads];
   __shared__ RefineQueue s_rq[kTraceWarps];
@@ -172,7 +186,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_any(const T
   };
   while (true) {
     uint32_t n;
-    if (take_rays<BATCHED>(A, active, drained, r, R, n, base_leaf, base_node)) {
+    if (take_rays<BATCHED, REFILL>(A, active, drained, r, R, n, base_leaf, base_node)) {
       active = true;
       best = kMiss;
       bt = R.tmax;
@@ -232,7 +246,7 @@ constexpr int kLeafFlush = 12;
 constexpr int kSteps = 6;  // node steps between two looks at what else is to be done
 constexpr int kLeafQueue = 96;  // a step queues at most 64
 
-template <bool BATCHED, bool V8>
+template <bool BATCHED, bool V8, int REFILL>
 __global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_closest(const TraceArgs A) {
   __shared__ float2 s_stack[kStackShared][kTraceThreads];
   __shared__ RefineQueue s_rq[kTraceWarps];
@@ -327,7 +341,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_closest(con
       uint32_t n;
       Ray R;
       bool one = false;
-      if (take_rays<BATCHED>(A, active, drained, r, R, n, base_leaf, base_node)) {
+      if (take_rays<BATCHED, REFILL>(A, active, drained, r, R, n, base_leaf, base_node)) {
         active = true;
         P = ray_pairs(R);
         bt = R.tmax;
@@ -382,7 +396,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_closest(con
     const bool done = W.node < 0;
     const unsigned waiting = __ballot_sync(FULL_MASK, done && active && pending);
     const unsigned running = __ballot_sync(FULL_MASK, active && !done);
-    if (nq >= kLeafFlush || (waiting && (!running || A.lanes - __popc(running) >= kTraceRefill))) flush();
+    if (nq >= kLeafFlush || (waiting && (!running || A.lanes - __popc(running) >= REFILL))) flush();
     const bool fin = active && done && !pending;
     if (__any_sync(FULL_MASK, fin)) {
       const bool hit = fin && (uint32_t)sbest[lane] != kMiss;
@@ -516,27 +530,32 @@ gprtcuStatus trace_launch(const gprtcuLbvh *bvh, const uint32_t *tri_off, const 
   a.counter = counter;
   a.err = &hdr->status;
   const bool v8 = ((uintptr_t)bvh->bvh2 & 31) == 0;
-#define GPRTCU_LAUNCH(K, CTAS, THREADS)                                 \
-  do {                                                                  \
-    if (meshes > 1) {                                                   \
-      if (v8) K<true, true><<<CTAS, THREADS, 0, stream>>>(a);           \
-      else K<true, false><<<CTAS, THREADS, 0, stream>>>(a);             \
-    } else {                                                            \
-      if (v8) K<false, true><<<CTAS, THREADS, 0, stream>>>(a);          \
-      else K<false, false><<<CTAS, THREADS, 0, stream>>>(a);            \
-    }                                                                   \
-  } while (0)
-#define GPRTCU_TRACE(K) GPRTCU_LAUNCH(K, g.ctas, kTraceThreads)
-  if (any) {
-    GPRTCU_TRACE(k_trace_any);
-  } else if (const RayGrid few = pool_grid(nrays); few.lanes) {
+  auto walk = [&](auto refill) {
+    constexpr int F = decltype(refill)::value;
+    auto launch = [&](auto kernel) { kernel<<<g.ctas, kTraceThreads, 0, stream>>>(a); };
+    if (any) v8 ? launch(k_trace_any<false, true, F>) : launch(k_trace_any<false, false, F>);
+    else v8 ? launch(k_trace_closest<false, true, F>) : launch(k_trace_closest<false, false, F>);
+  };
+  auto walk_batch = [&]() {
+    auto launch = [&](auto kernel) { kernel<<<g.ctas, kTraceThreads, 0, stream>>>(a); };
+    constexpr int F = kTraceRefill;
+    if (any) v8 ? launch(k_trace_any<true, true, F>) : launch(k_trace_any<true, false, F>);
+    else v8 ? launch(k_trace_closest<true, true, F>) : launch(k_trace_closest<true, false, F>);
+  };
+  if (const RayGrid few = pool_grid(nrays); !any && few.lanes) {
     a.lanes = few.lanes;
-    GPRTCU_LAUNCH(k_trace_pool, few.ctas, kPoolThreads);
+    auto launch = [&](auto kernel) { kernel<<<few.ctas, kPoolThreads, 0, stream>>>(a); };
+    if (meshes > 1) v8 ? launch(k_trace_pool<true, true>) : launch(k_trace_pool<true, false>);
+    else v8 ? launch(k_trace_pool<false, true>) : launch(k_trace_pool<false, false>);
+  } else if (meshes > 1) {
+    walk_batch();
   } else {
-    GPRTCU_TRACE(k_trace_closest);
+    switch (trace_refill(bvh->numPrims, meshes)) {
+      case 32: walk(std::integral_constant<int, 32>()); break;
+      case 24: walk(std::integral_constant<int, 24>()); break;
+      default: walk(std::integral_constant<int, kTraceRefill>()); break;
+    }
   }
-#undef GPRTCU_LAUNCH
-#undef GPRTCU_TRACE
   GPRTCU_TRY(cudaGetLastError());
   return GPRTCU_OK;
 }

@@ -63,6 +63,23 @@ def test_trace_overlapping(cuda, n, m):
     assert _same(api.hits_numpy(api.trace(b, torch.from_numpy(rays).cuda())), _expect(pos, tri, rays))
 
 
+@pytest.mark.parametrize("n", [5000000, 5000001, 12000001])
+@pytest.mark.parametrize("anyhit", [False, True])
+def test_trace_large_meshes(cuda, n, anyhit):
+    """The sizes at which a warp's refill changes; the hits of the quantised
+    traversal, whose code does not depend on the size."""
+    from gprt_b200 import api
+    pos, tri = api.gen_mixture(n, clusters=64, seed=9)
+    rays = api.gen_rays(200001, seed=10)
+    b = api.lbvh_build_triangles(pos, tri, api.Lbvh(n, with_aabbs=False))
+    hb = api.hits_numpy(api.trace(b, rays, anyhit=anyhit))
+    hw = api.hits_numpy(api.wide_trace(api.wide_build(b), rays, anyhit=anyhit))
+    if anyhit:
+        assert np.array_equal(hb["prim"] != 0xFFFFFFFF, hw["prim"] != 0xFFFFFFFF)
+    else:
+        assert np.array_equal(hb["prim"], hw["prim"]) and np.array_equal(hb["t"].view(np.uint32), hw["t"].view(np.uint32))
+
+
 @pytest.mark.parametrize("shift", [0, 16])
 def test_batch_trace_forms(cuda, shift):
     import torch
