@@ -779,13 +779,21 @@ __global__ void __launch_bounds__(kWideThreads, kWideCtas)
           if (isect_tri(Q, v0, v1, v2, t)) {
             key = ANY ? ((unsigned long long)(b + (int)(code & 31u)) << 32) | t_order(t)
                       : ((unsigned long long)t_order(t) << 32) | id;
-            atomicMin(&sbest[o], key);
+            if (!ANY) atomicMin(&sbest[o], key);
           }
+        }
+        unsigned long long before = 0;  // any hit: the key that s_bid belongs to
+        if constexpr (ANY) {
+          before = sbest[o];
+          __syncwarp();
+          if (key != ~0ull) atomicMin(&sbest[o], key);
         }
         __syncwarp();
         bool won = key != ~0ull && sbest[o] == key;
-        if constexpr (ANY) {  // the same entry and distance: the lowest id
-          if (won) s_bid[wq][o] = kMiss;
+        if constexpr (ANY) {
+          // the same entry and distance: the lowest id, over all 32-test
+          // batches that the entry's tests are in
+          if (won && before != key) s_bid[wq][o] = kMiss;
           __syncwarp();
           if (won) atomicMin(&s_bid[wq][o], id);
           __syncwarp();

@@ -225,3 +225,31 @@ def test_wide_closest_ties_and_zero_t(cuda):
     n_extra = len(extra)
     assert (gw["prim"][-n_extra:] != 0xFFFFFFFF).all()
     assert (gw["t"][-n_extra::3] == 0.0).all() and (gw["t"][-n_extra + 1::3] == 0.0).all()
+
+
+@pytest.mark.parametrize("n", [3, 5, 7, 8])
+def test_wide_any_ties(cuda, n):
+    """Any hit over coincident triangles, all children of one node: the lowest
+    id of those at the same distance, wherever the 32-test batches of a warp's
+    queue divide the node's tests (rays that miss some or all of them shift
+    the division)."""
+    import torch
+    from gprt_b200 import api
+    rng = np.random.default_rng(n)
+    one = np.float32([[0.0, 0.0, 0.0], [1.0, 0.0, 0.0], [0.0, 1.0, 0.0]])
+    pos = np.tile(one, (n, 1))
+    tri = np.arange(3 * n, dtype=np.uint32).reshape(n, 3)
+    m = 20011
+    rays = np.zeros((m, 8), np.float32)
+    rays[:, :2] = rng.random((m, 2)) * 0.7
+    rays[:, 2] = -1.0
+    rays[:, 6] = 1.0
+    rays[:, 7] = np.inf
+    inside = rays[:, 0] + rays[:, 1] < 1.0
+    b = api.lbvh_build_triangles(torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda())
+    w = api.wide_build(b)
+    assert api.wide_decode(w)["count"] == 1
+    r = torch.from_numpy(rays).cuda()
+    for _ in range(5):
+        h = api.hits_numpy(api.wide_trace(w, r, anyhit=True))
+        assert np.array_equal(h["prim"], np.where(inside, 0, 0xFFFFFFFF).astype(np.uint32))
