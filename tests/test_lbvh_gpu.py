@@ -238,3 +238,28 @@ def test_refit_after_moving_vertices(cuda, n):
     got = api.hits_numpy(api.trace(bvh, torch.from_numpy(rays).cuda()))
     exp = oracle.trace_brute(moved, tri, rays)
     assert np.array_equal(got["prim"], exp["prim"])
+
+
+@pytest.mark.parametrize("n", [100_001, 500_001])
+def test_refit_takes_less_than_a_build(cuda, n):
+    """A refit is a part of a build (no bounds, codes, sort or topology), so
+    its time stays below the build's."""
+    import torch
+    from gprt_b200 import api
+    pos, tri = api.gen_soup(n, seed=n)
+    b = api.Lbvh(n)
+
+    def us(f):
+        times = []
+        for _ in range(12):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            f()
+            e[1].record()
+            e[1].synchronize()
+            times.append(e[0].elapsed_time(e[1]))
+        return 1e3 * sorted(times[2:])[5]
+
+    build = us(lambda: api.lbvh_build_triangles(pos, tri, b))
+    refit = us(lambda: api.lbvh_refit_triangles(pos, tri, b))
+    assert refit < build, (refit, build)
