@@ -87,7 +87,7 @@ struct Walk {
   __device__ __forceinline__ void start() {
     node = 0;
     top = kWalkEnd;
-    t = top_t = 0.0f;
+    t = top_t = -INFINITY;  // the root is visited whatever the ray's range
     sp = 0;
   }
 };
@@ -228,7 +228,7 @@ __device__ __forceinline__ bool pool_walk(PoolShared &S, const Bvh2Node *bvh, bo
     __syncwarp();
   };
   __syncwarp();
-  push(root, root ? (int)S.base[lane][1] : 0, 0.0f, lane);
+  push(root, root ? (int)S.base[lane][1] : 0, -INFINITY, lane);
   queue(one, one ? S.base[lane][0] : 0u, lane);
   while (true) {
     __syncwarp();

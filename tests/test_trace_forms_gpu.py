@@ -318,3 +318,35 @@ def test_wide_forms(cuda, n, m, shift):
     assert _same(api.hits_numpy(api.wide_trace(w, rays)), exp)
     anyh = api.hits_numpy(api.wide_trace(w, rays, anyhit=True))
     assert np.array_equal(anyh["prim"] != 0xFFFFFFFF, exp["prim"] != 0xFFFFFFFF)
+
+
+@pytest.mark.parametrize("m", [300, 4099, 200003])
+def test_ranges_behind_the_origin(cuda, m):
+    """Rays whose whole range [tmin, tmax] is negative: the closest hit is
+    looked for as any hit is."""
+    import torch
+    from gprt_b200 import api
+    n = 700
+    pos, tri = scenes.soup(n, seed=1, sigma=0.05)
+    rays = scenes.rays(m, seed=m)
+    rays[:, 4:7] *= -1.0
+    rays[:, 3] = -4.0
+    rays[:, 7] = -0.125
+    p, t, r = torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda(), torch.from_numpy(rays).cuda()
+    b = api.lbvh_build_triangles(p, t)
+    exp = _expect(pos, tri, rays)
+    hit = exp["prim"] != 0xFFFFFFFF
+    assert hit.sum() > m // 10
+    assert _same(api.hits_numpy(api.trace(b, r)), exp)
+    assert np.array_equal(api.hits_numpy(api.trace(b, r, anyhit=True))["prim"] != 0xFFFFFFFF, hit)
+    rec = np.zeros(3, np.dtype(api.INSTANCE_DTYPE))
+    rec["transform"][:, [0, 5, 10]] = 1.0
+    rec["transform"][:, 3] = [0.0, 50.0, 100.0]
+    rec["custom_mask"] = 0xFF << 24
+    h, i = api.trace_instances(api.Tlas(api.instances_tensor(rec), b.root, 1), b, r)
+    assert np.array_equal(api.hits_numpy(h)["prim"], exp["prim"])
+    sph = np.concatenate([np.random.default_rng(2).random((n, 3)), np.full((n, 1), 0.03)], 1).astype(np.float32)
+    s = torch.from_numpy(sph).cuda()
+    got = api.hits_numpy(api.trace_spheres(api.lbvh_build_boxes(api.sphere_bounds(s)), s, r))
+    e = oracle.trace_user_brute(0, sph, rays)
+    assert np.array_equal(got["prim"], e["prim"]) and (e["prim"] != 0xFFFFFFFF).sum() > m // 10
