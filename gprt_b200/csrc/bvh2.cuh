@@ -54,20 +54,24 @@ __device__ __forceinline__ RayPairs ray_pairs(const Ray &r) {
   return RayPairs{pk2(-r.ox, -r.oy), pk2(-r.oz, -r.oz), pk2(r.ix, r.iy), pk2(r.iz, r.iz), r.tmin};
 }
 
-// ray_box with the result in one word: the child's entry distance, or NaN
-// when it is not to be entered, i.e. unless ray_box(..., bt, tn) && tn <= bt.
+// ray_box(..., bt, tn) && tn <= bt of a child's box, bt being a number.
 // The exit is widened before it is clamped by bt, which is the same test:
 // entry <= min(exit, bt) x kBoxHi and entry <= bt hold together exactly when
 // entry <= min(exit x kBoxHi, bt), bt being no less than zero.
-__device__ __forceinline__ float child_entry(const ChildPairs &n, const RayPairs &r, float bt) {
+__device__ __forceinline__ bool child_hit(const ChildPairs &n, const RayPairs &r, float bt, float &tn) {
   float x0, y0, z0, x1, y1, z1;
   up2(mul2_rn(add2_rn(n.b[0], r.nxy), r.ixy), x0, y0);
   up2(mul2_rn(add2_rn(n.b[1], r.nxy), r.ixy), x1, y1);
   up2(mul2_rn(add2_rn(n.b[2], r.nzz), r.izz), z0, z1);
-  const float tn =
-      __fmul_rn(fmaxf(max3f(nan_min(x0, x1), nan_min(y0, y1), nan_min(z0, z1)), r.tmin), kBoxLo);
+  tn = __fmul_rn(fmaxf(max3f(nan_min(x0, x1), nan_min(y0, y1), nan_min(z0, z1)), r.tmin), kBoxLo);
   const float tf = __fmul_rn(min3f(nan_max(x0, x1), nan_max(y0, y1), nan_max(z0, z1)), kBoxHi);
-  return tn <= fminf(tf, bt) ? tn : __int_as_float(0x7fffffff);
+  return tn <= fminf(tf, bt);
+}
+// The same in one word: the child's entry distance, or NaN when it is not to
+// be entered.
+__device__ __forceinline__ float child_entry(const ChildPairs &n, const RayPairs &r, float bt) {
+  float tn;
+  return child_hit(n, r, bt, tn) ? tn : __int_as_float(0x7fffffff);
 }
 
 // A lane's walk over the tree: its node (negative: the walk is over) with the
@@ -91,9 +95,6 @@ struct Walk {
     sp = 0;
   }
 };
-// Moves on: t0, t1 are the entry distances of the children (NaN: not to be
-// entered) of the lane's node, on whether it has one.  Returns false when the
-// stack is full.
 // Puts (node, t) on top of the stack; false when it is full.
 template <int THREADS, int SHARED, int DEPTH>
 __device__ __forceinline__ bool walk_push(Walk &W, float2 *sh, float2 *over, int node, float t) {
@@ -116,6 +117,10 @@ __device__ __forceinline__ void walk_pop(Walk &W, const float2 *sh, const float2
   W.top = W.sp < 0 ? kWalkEnd : __float_as_int(e.x);
   W.top_t = e.y;
 }
+// Moves on: t0, t1 are the entry distances of the children (NaN: not to be
+// entered) of the lane's node, on whether it has one; a lane without one
+// passes NaN twice.  Returns false when the stack is full: the walk is then
+// over, and the caller sets W.node to the end.
 template <int THREADS, int SHARED, int DEPTH>
 __device__ __forceinline__ bool walk_next(Walk &W, float2 *sh, float2 *over, bool on, float t0, int r0, float t1,
                                           int r1) {
@@ -145,9 +150,11 @@ __device__ __forceinline__ bool walk_next(Walk &W, float2 *sh, float2 *over, boo
 // a time.  A ray's chain is then its depth plus its share of the warp's visits
 // divided by 32.  Whole calls, lane per ray / pooled: 4,099 rays on 1,501
 // triangles 80 / 30 us, on 262,144 triangles 210 / 38 us; 40,001 rays there
-// 348 / 156 us, 113,001 403 / 362 us; from there the lane per ray is faster
-// (200,001: 558 / 627 us; 1,048,576: 1.94 / 2.9 ms), since nearer nodes are not
-// strictly first and every step reads its ray from shared memory.  The closest
+// 348 / 156 us.  With more rays the lane per ray is faster (1,048,576: 1.94 /
+// 2.9 ms), since nearer nodes are not strictly first (twice the visits on dense
+// primitives) and every step reads its ray from shared memory; from how many
+// on depends on what a test costs and how deep the tree is, so the callers
+// give the line (pool_grid).  The closest
 // (t, id) is the same in any order.  Where boxes overlap so much that nearly
 // every child is entered, the stack grows to the lanes times the tree's depth;
 // from kPoolWide entries on, fewer lanes go on the fuller it is (an eighth of
@@ -161,7 +168,6 @@ constexpr int kPoolLeaves = 96;              // a step queues at most 64
 constexpr int kPoolThreads = 64;
 constexpr int kPoolWarps = kPoolThreads / 32;
 constexpr int kPoolCtas = 12;
-constexpr int kPoolRounds = 2;  // chunks of kPoolRays per warp up to which rays are few
 
 struct PoolShared {
   uint2 stack[kPoolStack];  // node, entry distance
@@ -304,10 +310,10 @@ __device__ __forceinline__ bool warp_take(bool active, bool &drained, int lanes,
 // instead, at least four to each (a warp's time is that of its longest ray,
 // and lanes without a ray still run queued primitive tests).  4,099 rays on
 // 1,501 triangles at 32 / 16 / 8 / 4 / 2 / 1 rays per warp: 102 / 85 / 81 / 78
-// / 78 / 93 us.  Spread over every warp that fits (32 per SM) the warps' own
-// instructions add up: 18,001 rays on 262,144 triangles, any hit, 335 us
-// against 272 us.
-constexpr int kSpreadWarps = 8;
+// / 78 / 93 us.  8 / 12 / 16 / 24 warps per SM: any hit of 25,001 rays on 2,657
+// triangles 58.4 / 57.6 / 55.5 / 57.9 us, of 56,001 on 20,001 triangles 130 /
+// 130 / 131 / 137 us, of 40,001 on 4.2 M triangles 1,063 / 960 / 917 / 908 us.
+constexpr int kSpreadWarps = 16;
 struct RayGrid {
   int ctas, lanes;
 };
@@ -320,10 +326,11 @@ static inline RayGrid ray_grid(uint64_t nrays, int ctas, int warps) {
   return RayGrid{(int)(need < fit ? need : fit), lanes};
 }
 // Grid of a pool kernel and the rays a warp takes at a time (two at least); 0
-// rays when there are too many for it.
-static inline RayGrid pool_grid(uint64_t nrays) {
+// rays when there are more than `sixths` sixths of a chunk of kPoolRays for
+// every warp that fits.
+static inline RayGrid pool_grid(uint64_t nrays, int sixths) {
   const uint64_t fit = (uint64_t)gprtcu_num_sms() * gprtcu::kPoolCtas, warps = fit * gprtcu::kPoolWarps;
-  if (nrays > warps * gprtcu::kPoolRays * gprtcu::kPoolRounds) return RayGrid{0, 0};
+  if (6 * nrays > warps * gprtcu::kPoolRays * sixths) return RayGrid{0, 0};
   const uint64_t share = (nrays + warps - 1) / warps;
   const int lanes = share > gprtcu::kPoolRays ? gprtcu::kPoolRays : (share < 2 ? 2 : (int)share);
   const uint64_t need = (nrays + (uint64_t)lanes * gprtcu::kPoolWarps - 1) / ((uint64_t)lanes * gprtcu::kPoolWarps);

@@ -122,7 +122,10 @@ __device__ __forceinline__ void finish_rays(const TraceArgs &A, RefineQueue &q, 
 // Idle lanes take new rays (warp_take).  Returns true on the lanes that took
 // one; base_leaf and base_node are the first leaf slot and node of the ray's
 // mesh and n its triangles.
-constexpr int kTraceRefill = 8;
+// Rays beyond the 151,552 that 148 SMs hold at once start as soon as this many
+// of a warp's lanes are idle: at 8 / 4 lanes 185,001 rays on 5,001 triangles
+// take 160 / 156 us.
+constexpr int kTraceRefill = 4;
 // One mesh whose nodes and leaves (112 bytes a triangle) pass some 560 MB: a
 // node that is not in L2 costs so much more from there on that rays which
 // start together are worth more than full lanes, since they meet in the upper
@@ -131,9 +134,12 @@ constexpr int kTraceRefill = 8;
 // M 13.5 / 11.6 / 15.6, 8.4 M 25.5 / 21.2 / 23.2; 4.2 M rays on 16.8 M
 // triangles 66 / 56 / 52 ms, on 33.6 M 18.5 / 15.8 / 15.5 (any hit alike).
 // The meshes of a batch are small, and a warp's rays are of one or two.
-// (An argument instead of a template parameter cost 3 %.)
-static inline int trace_refill(uint32_t n, uint32_t meshes) {
-  if (meshes > 1 || n <= 5000000u) return kTraceRefill;
+// (An argument instead of a template parameter cost 3 %.)  Calls with fewer
+// rays than the GPU holds at once hardly refill and do not mind: 130,001 rays
+// on 16.8 M triangles 2.76 ms with 32, 2.72 ms with 4; 400,001 6.45 against
+// 7.13 ms.
+static inline int trace_refill(uint32_t n) {
+  if (n <= 5000000u) return kTraceRefill;
   return n <= 12000000u ? 24 : 32;
 }
 
@@ -154,31 +160,62 @@ __device__ __forceinline__ bool take_rays(const TraceArgs &A, bool active, bool 
   return true;
 }
 
-// Any hit: a lane tests the leaf triangles it meets at once, and the first
-// step with a hit ends its ray.
+// Any hit: a lane tests the leaf triangles it meets at once, child 0 first,
+// and the first step with a hit ends its ray (so the hit is the first of the
+// near-first order, however the rays share warps).  Few rays wait for a chain
+// of visits, so what a visit costs besides its load counts: votes for new and
+// finished rays are taken every kAnySteps visits (at every visit: 2,657
+// triangles and 56,001 rays 71.4 us, 4.2 M triangles and 4.0 M rays 16.8 ms;
+// now 65.5 us, 15.1 ms), the stack holds nodes alone since nothing is culled
+// by distance, and with few rays 16 instead of 8 warps per SM share them
+// (ray_grid; 40,001 rays on 4.2 M triangles 1,122 -> 911 us).  1,000,001 rays
+// on 100,001 triangles: votes at every / 2nd / 4th / 8th visit 1,564 / 1,553 /
+// 1,540 / 1,538 us; then nodes alone on the stack 1,470, every 12th visit 1,464
+// us.  10 CTAs per SM spill: 1,547 us.  Stack entries in shared memory 12 / 6 /
+// 3: 1,461 / 1,474 / 1,547 us.
+constexpr int kAnySteps = 12;
+constexpr int kAnyCtas = 8;
+constexpr int kAnyShared = 12;  // stack entries in shared memory
 template <bool BATCHED, bool V8, int REFILL>
-__global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_any(const TraceArgs A) {
-  __shared__ float2 s_stack[kStackShared][kTraceThreads];
+__global__ void __launch_bounds__(kTraceThreads, kAnyCtas) k_trace_any(const TraceArgs A) {
+  __shared__ int s_stack[kAnyShared][kTraceThreads];
   __shared__ RefineQueue s_rq[kTraceWarps];
   RefineQueue &rq = s_rq[threadIdx.x >> 5];
   bool active = false, drained = false;
   uint64_t r = 0;
-  Ray R;
+  RayPairs P;
+  P.nxy = P.nzz = P.ixy = P.izz = 0;
+  P.tmin = 0.0f;
+  float Sx = 0.0f, Sy = 0.0f, Sz = 0.0f, tmax = 0.0f;
+  int axes = 0;  // kx | ky << 2 | kz << 4
   uint32_t base_leaf = 0, base_node = 0, best = kMiss, best_slot = 0;
   float bt = 0.0f;
   int nrq = 0;
-  Walk W;
-  W.start();
-  W.node = -1;
-  float2 *const sh = &s_stack[0][threadIdx.x];
-  float2 over[kStackDepth - kStackShared];
+  int node = -1, top = -1, sp = 0;  // the walk: its node, the stack's top entry and the entries below it
+  int *const sh = &s_stack[0][threadIdx.x];
+  int over[kStackDepth - kAnyShared];
   auto leaf_test = [&](uint32_t slot) {
+    Ray Q;
+    float nx, ny, nz, unused;
+    up2(P.nxy, nx, ny);
+    up2(P.nzz, nz, unused);
+    Q.ox = -nx;
+    Q.oy = -ny;
+    Q.oz = -nz;
+    Q.tmin = P.tmin;
+    Q.tmax = tmax;
+    Q.Sx = Sx;
+    Q.Sy = Sy;
+    Q.Sz = Sz;
+    Q.kx = axes & 3;
+    Q.ky = (axes >> 2) & 3;
+    Q.kz = axes >> 4;
     const float4 a = __ldg(A.leaf + 3 * (size_t)slot), b = __ldg(A.leaf + 3 * (size_t)slot + 1),
                  c = __ldg(A.leaf + 3 * (size_t)slot + 2);
     const float v0[3] = {a.x, a.y, a.z}, v1[3] = {b.x, b.y, b.z}, v2[3] = {c.x, c.y, c.z};
     const uint32_t id = __float_as_uint(a.w);
     float t;
-    if (isect_tri(R, v0, v1, v2, t) && (best == kMiss || t < bt || (t == bt && id < best))) {
+    if (isect_tri(Q, v0, v1, v2, t) && (best == kMiss || t < bt || (t == bt && id < best))) {
       best = id;
       best_slot = slot;
       bt = t;
@@ -186,38 +223,61 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_any(const T
   };
   while (true) {
     uint32_t n;
+    Ray R;
     if (take_rays<BATCHED, REFILL>(A, active, drained, r, R, n, base_leaf, base_node)) {
       active = true;
       best = kMiss;
-      bt = R.tmax;
-      W.start();
+      P = ray_pairs(R);
+      Sx = R.Sx;
+      Sy = R.Sy;
+      Sz = R.Sz;
+      axes = R.kx | (R.ky << 2) | (R.kz << 4);
+      bt = tmax = R.tmax;
+      node = bt == bt ? 0 : -1;  // no box lies in a range that ends in NaN
+      top = -1;
+      sp = 0;
       if (n == 1) {
         if (single_leaf_box(A.leaf, base_leaf, R)) leaf_test(base_leaf);
-        W.node = -1;
+        node = -1;
       }
     }
     if (!__any_sync(FULL_MASK, active)) {
       if (drained) break;
       continue;
     }
-    if (W.node >= 0) {
-      const Bvh2Node *nd = A.bvh + base_node + W.node;
-      const ChildPairs c0 = load_child<V8>(&nd->c[0]), c1 = load_child<V8>(&nd->c[1]);
-      const RayPairs P = ray_pairs(R);
-      float t0 = child_entry(c0, P, bt), t1 = child_entry(c1, P, bt);
-      const bool leaf0 = c0.ref < 0 && t0 == t0, leaf1 = c1.ref < 0 && t1 == t1;
-      if (leaf0) leaf_test(base_leaf + (uint32_t)~c0.ref);
-      if (leaf1 && t1 <= bt) leaf_test(base_leaf + (uint32_t)~c1.ref);
-      if (c0.ref < 0) t0 = __int_as_float(0x7fffffff);
-      if (c1.ref < 0) t1 = __int_as_float(0x7fffffff);
-      if (best != kMiss) {
-        W.node = -1;
-      } else if (!walk_next<kTraceThreads, kStackShared, kStackDepth>(W, sh, over, true, t0, c0.ref, t1, c1.ref)) {
-        atomicCAS(A.err, 0u, 5u);  // traversal stack overflow
-        W.node = -1;
+#pragma unroll 1
+    for (int step = 0; step < kAnySteps; ++step) {
+      if (node >= 0) {
+        const Bvh2Node *nd = A.bvh + base_node + node;
+        const ChildPairs c0 = load_child<V8>(&nd->c[0]), c1 = load_child<V8>(&nd->c[1]);
+        float t0, t1;
+        const bool h0 = child_hit(c0, P, bt, t0), h1 = child_hit(c1, P, bt, t1);
+        if (h0 && c0.ref < 0) leaf_test(base_leaf + (uint32_t)~c0.ref);
+        if (h1 && c1.ref < 0 && t1 <= bt) leaf_test(base_leaf + (uint32_t)~c1.ref);
+        const bool in0 = h0 && c0.ref >= 0, in1 = h1 && c1.ref >= 0;
+        const bool first = in0 && !(in1 && t1 < t0);  // the nearer child, child 0 on ties
+        if (best != kMiss) {
+          node = -1;
+        } else if (in0 || in1) {
+          if (in0 && in1) {
+            if (sp < kAnyShared) sh[sp * kTraceThreads] = top;
+            else if (sp < kStackDepth) over[sp - kAnyShared] = top;
+            ++sp;
+            top = first ? c1.ref : c0.ref;
+          }
+          node = first ? c0.ref : c1.ref;
+          if (sp > kStackDepth) {
+            atomicCAS(A.err, 0u, 5u);  // traversal stack overflow
+            node = -1;
+          }
+        } else {
+          node = top;
+          --sp;
+          top = sp < 0 ? -1 : (sp < kAnyShared ? sh[sp * kTraceThreads] : over[sp - kAnyShared]);
+        }
       }
     }
-    const bool fin = active && W.node < 0;
+    const bool fin = active && node < 0;
     if (__any_sync(FULL_MASK, fin)) {
       finish_rays(A, rq, nrq, fin, best != kMiss, r, best_slot);
       if (fin) active = false;
@@ -239,11 +299,15 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_any(const T
 // 77.5 M rays over 4,096 meshes 48.5 -> 31.6 ms.  Flush at 8 / 12 / 16 / 20 /
 // 24 tests: 1.91 / 1.93 / 1.94 / 1.96 / 2.03 ms; 1 / 2 / 4 / 6 / 8 node steps
 // between two looks at refill, flush and finished rays: 2.08 / 2.05 / 1.93 /
-// 1.92 / 2.10 ms.  Shared memory decides how much of it L1 keeps: 18 KB per
-// CTA at 8 CTAs leaves 64 KB; 22 KB at 9 CTAs leaves next to none, and the
-// 4.2 M triangles took 11.7 ms.
+// 1.92 / 2.10 ms.  Once there are no more rays to take, a warp's time is that
+// of its longest ray, and the looks are part of it: 6 / 10 / 16 / 24 steps from
+// then on take 146 / 143 / 142 / 143 us for 170,001 rays on 5,001 triangles.
+// Shared memory decides how much of it L1 keeps: 18 KB per CTA at 8 CTAs leaves
+// 64 KB; 22 KB at 9 CTAs leaves next to none, and the 4.2 M triangles took 11.7
+// ms.
 constexpr int kLeafFlush = 12;
 constexpr int kSteps = 6;  // node steps between two looks at what else is to be done
+constexpr int kStepsLast = kSteps;  // the same, once there are no more rays to take
 constexpr int kLeafQueue = 96;  // a step queues at most 64
 
 template <bool BATCHED, bool V8, int REFILL>
@@ -366,7 +430,7 @@ __global__ void __launch_bounds__(kTraceThreads, kTraceCtas) k_trace_closest(con
       queue(one, base_leaf);
     }
 #pragma unroll 1
-    for (int step = 0; step < kSteps; ++step) {
+    for (int step = 0; step < (drained ? kStepsLast : kSteps); ++step) {
       const bool on = W.node >= 0;
       float t0 = __int_as_float(0x7fffffff), t1 = t0;
       int r0 = 0, r1 = 0;
@@ -542,7 +606,8 @@ gprtcuStatus trace_launch(const gprtcuLbvh *bvh, const uint32_t *tri_off, const 
     if (any) v8 ? launch(k_trace_any<true, true, F>) : launch(k_trace_any<true, false, F>);
     else v8 ? launch(k_trace_closest<true, true, F>) : launch(k_trace_closest<true, false, F>);
   };
-  if (const RayGrid few = pool_grid(nrays); !any && few.lanes) {
+  const int pool_sixths = 12;
+  if (const RayGrid few = pool_grid(nrays, pool_sixths); !any && few.lanes) {
     a.lanes = few.lanes;
     auto launch = [&](auto kernel) { kernel<<<few.ctas, kPoolThreads, 0, stream>>>(a); };
     if (meshes > 1) v8 ? launch(k_trace_pool<true, true>) : launch(k_trace_pool<true, false>);
@@ -550,7 +615,7 @@ gprtcuStatus trace_launch(const gprtcuLbvh *bvh, const uint32_t *tri_off, const 
   } else if (meshes > 1) {
     walk_batch();
   } else {
-    switch (trace_refill(bvh->numPrims, meshes)) {
+    switch (trace_refill(bvh->numPrims)) {
       case 32: walk(std::integral_constant<int, 32>()); break;
       case 24: walk(std::integral_constant<int, 24>()); break;
       default: walk(std::integral_constant<int, kTraceRefill>()); break;

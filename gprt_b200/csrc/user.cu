@@ -230,7 +230,7 @@ __device__ __forceinline__ bool odd_key(unsigned long long key) { return (uint32
 __device__ __forceinline__ unsigned long long hit_key(float t, uint32_t id) {
   return t == t ? ((unsigned long long)t_order(t) << 32) | id : kOddKey;
 }
-template <typename PRIMS> __device__ __forceinline__ void user_odd(const UserArgs<PRIMS> &A, uint64_t r, bool any) {
+template <typename PRIMS> __device__ __forceinline__ void user_odd(const UserArgs<PRIMS> &A, uint64_t r) {
   Ray R;
   ray_setup(__ldg(A.rays + 2 * r), __ldg(A.rays + 2 * r + 1), R);
   uint32_t best = kMiss;
@@ -261,7 +261,6 @@ template <typename PRIMS> __device__ __forceinline__ void user_odd(const UserArg
     if (h0 && r0 < 0) leaf((uint32_t)~r0);
     h1 = h1 && tn1 <= bt;
     if (h1 && r1 < 0) leaf((uint32_t)~r1);
-    if (any && best != kMiss) break;
     h0 = h0 && r0 >= 0;
     h1 = h1 && r1 >= 0 && tn1 <= bt;
     if (h0 && h1) {
@@ -312,13 +311,13 @@ __device__ __forceinline__ void user_hit(const UserArgs<PRIMS> &A, uint64_t r, u
   if (A.hit_u) A.hit_u[r] = hit ? u : 0.0f;
 }
 template <typename PRIMS>
-__device__ __forceinline__ void user_odds(const UserArgs<PRIMS> &A, float2 odd, bool any) {
+__device__ __forceinline__ void user_odds(const UserArgs<PRIMS> &A, float2 odd) {
   while (true) {
     const uint64_t r = ((unsigned long long)__float_as_uint(odd.y) << 32) | __float_as_uint(odd.x);
     if (r == kOddEnd) break;
     const Hit h = A.hits[r];
     odd = make_float2(__uint_as_float(h.prim), h.t);
-    user_odd(A, r, any);
+    user_odd(A, r);
   }
 }
 
@@ -326,17 +325,21 @@ __device__ __forceinline__ void user_odds(const UserArgs<PRIMS> &A, float2 odd, 
 // test at the leaves: leaf slot s holds primitive ids[s].  One lane per ray,
 // refilled as rays finish.  Closest hit queues the tests of the leaf children
 // it meets per warp as (slot, lane) and runs them with all lanes, each folding
-// its hit into the owner's (t, id) key; any hit tests them at once, the first
-// step with a hit ending the ray.  (A test is 150 to 200 instructions; run
+// its hit into the owner's (t, id) key.  (A test is 150 to 200 instructions; run
 // where the walk met them, with whole warps waiting for their longest ray,
 // they left 8.4 of 32 lanes active.  1,048,577 rays on 1,048,576 swept
-// spheres: 2.53 -> 1.47 ms closest, 2.40 -> 1.67 ms any; what bounds it now
-// is load latency with 28 warps per SM and L1's data pipe, 66 % busy.  Flush
-// at 8 / 12 / 24 / 32 tests: 1.56 / 1.56 / 1.60 / 1.66 ms, and from there 6 /
-// 8 / 10 node steps between two looks at flush and refill with 8 / 8 / 12
-// stack entries in shared memory: 1.56 / 1.52 / 1.47 ms.)
-template <typename PRIMS, bool ANY, bool V8>
-__global__ void __launch_bounds__(kUserThreads, kUserCtas) k_trace_user(const UserArgs<PRIMS> A) {
+// spheres: 2.51 -> 1.45 ms; what bounds it now is load latency and L1's data
+// pipe.  Flush at 8 / 12 / 24 / 32 tests: 1.56 / 1.56 / 1.60 / 1.66 ms, and from
+// there 6 / 8 / 10 node steps between two looks at flush and refill with 8 / 8 /
+// 12 stack entries in shared memory: 1.56 / 1.52 / 1.47 ms.)  With no more rays
+// to take, a flush comes as soon as the lanes still walking have a test each:
+// the culling distance lags less, which is worth more than full lanes then
+// (130,001 rays on 1,000,001 spheres 549 -> 481 us; 500 in the plain walk).  6 /
+// 7 / 8 CTAs per SM (80 / 72 / 64 registers, the last spilling 48 bytes): 1.47 /
+// 1.45 / 1.53 ms on the swept spheres above, 1.43 / 1.37 / 1.51 ms on as many
+// spheres; 10 / 14 node steps between two looks then 1.47 / 1.45 ms.
+template <typename PRIMS, bool V8>
+__global__ void __launch_bounds__(kUserThreads, kUserCtas) k_user_closest(const UserArgs<PRIMS> A) {
   __shared__ float2 s_stack[kUserShared][kUserThreads];
   __shared__ uint32_t s_qslot[kUserWarps][kUserQueue];
   __shared__ uint8_t s_qlane[kUserWarps][kUserQueue];
@@ -379,17 +382,6 @@ __global__ void __launch_bounds__(kUserThreads, kUserCtas) k_trace_user(const Us
     float t;
     if (!A.prims.hit(Q, id, A.exit_test, t, u)) return ~0ull;
     return hit_key(t, id);
-  };
-  auto test_now = [&](uint32_t slot) {  // any hit
-    float nx, ny, nz, unused, u;
-    up2(P.nxy, nx, ny);
-    up2(P.nzz, nz, unused);
-    const unsigned long long key = test(slot, lane, -nx, -ny, -nz, P.tmin, u);
-    if (key < s_best[tid]) {
-      s_best[tid] = key;
-      s_u[tid] = u;
-      bt = t_from_order((uint32_t)(key >> 32));
-    }
   };
   // every queued test by all lanes (warp-uniform call)
   auto flush = [&]() {
@@ -455,19 +447,15 @@ __global__ void __launch_bounds__(kUserThreads, kUserCtas) k_trace_user(const Us
         if (drained) break;
         continue;
       }
-      if (ANY) {
-        if (one) test_now(0);
-      } else {
-        if (nq > kUserQueue - 32) flush();
-        queue(one, 0u);
-      }
+      if (nq > kUserQueue - 32) flush();
+      queue(one, 0u);
     }
 #pragma unroll 1
     for (int step = 0; step < kUserSteps; ++step) {
       const bool on = W.node >= 0;
       float t0 = kNone, t1 = kNone;
       int r0 = 0, r1 = 0;
-      bool leaf0 = false, leaf1 = false, found = false;
+      bool leaf0 = false, leaf1 = false;
       if (on && W.t <= bt) {
         const Bvh2Node *nd = A.bvh + W.node;
         const ChildPairs c0 = load_child<V8>(&nd->c[0]), c1 = load_child<V8>(&nd->c[1]);
@@ -477,11 +465,6 @@ __global__ void __launch_bounds__(kUserThreads, kUserCtas) k_trace_user(const Us
         r1 = c1.ref;
         leaf0 = r0 < 0 && t0 == t0;
         leaf1 = r1 < 0 && t1 == t1;
-        if (ANY) {
-          if (leaf0) test_now((uint32_t)~r0);
-          if (leaf1 && t1 <= bt) test_now((uint32_t)~r1);
-          found = (leaf0 || leaf1) && (uint32_t)s_best[tid] != kMiss;
-        }
         if (leaf0) t0 = kNone;
         if (leaf1) t1 = kNone;
       }
@@ -489,25 +472,139 @@ __global__ void __launch_bounds__(kUserThreads, kUserCtas) k_trace_user(const Us
         atomicCAS(A.err, 0u, 5u);  // traversal stack overflow
         W.node = kWalkEnd;
       }
-      if (ANY && found) W.node = kWalkEnd;
-      if (!ANY && __any_sync(FULL_MASK, leaf0 || leaf1)) {
+      if (__any_sync(FULL_MASK, leaf0 || leaf1)) {
         if (nq > kUserQueue - 64) flush();
         queue(leaf0, (uint32_t)~r0);
         queue(leaf1, (uint32_t)~r1);
       }
     }
     const bool done = W.node == kWalkEnd;
-    if (!ANY) {
-      const unsigned waiting = __ballot_sync(FULL_MASK, done && active && pending);
-      const unsigned running = __ballot_sync(FULL_MASK, active && !done);
-      if (nq >= kUserFlush || (waiting && (!running || A.lanes - __popc(running) >= kUserRefill))) flush();
-    }
+    const unsigned waiting = __ballot_sync(FULL_MASK, done && active && pending);
+    const unsigned running = __ballot_sync(FULL_MASK, active && !done);
+    if (nq >= kUserFlush ||
+        (waiting && (!running || A.lanes - __popc(running) >= kUserRefill)))
+      flush();
     if (active && done && !pending) {
       user_hit(A, s_rid[tid], s_best[tid], s_u[tid], odd);
       active = false;
     }
   }
-  user_odds(A, odd, ANY);
+  user_odds(A, odd);
+}
+
+// Any hit: the primitives of the leaf children that a step meets are tested
+// at once, child 0 first, and the first step with a hit ends the ray, as the
+// any-hit walk over triangles does.  Ray and hit in registers and a stack of
+// nodes alone (the closest-hit kernel with its tests at once kept them in
+// shared memory, 17 KB a CTA): 30,001 / 1,000,001 rays on 1,000,001 swept
+// spheres 344 / 1,697 -> 317 / 1,504 us, 150,001 rays on 10,001 spheres 149 ->
+// 122 us.  Steps between two votes 12 / 12 and 48 once there are no more
+// rays to take: 20,001 rays on 1,001 spheres 29 / 33 us.
+constexpr int kUserAnyCtas = 8;
+constexpr int kUserAnyShared = 8;  // stack entries (nodes alone: nothing is culled by distance) in shared memory
+constexpr int kUserAnySteps = 12;
+template <typename PRIMS, bool V8>
+__global__ void __launch_bounds__(kUserThreads, kUserAnyCtas) k_user_any(const UserArgs<PRIMS> A) {
+  __shared__ int s_stack[kUserAnyShared][kUserThreads];
+  bool active = false, drained = false;
+  uint64_t r = 0;
+  RayPairs P;
+  P.nxy = P.nzz = P.ixy = P.izz = 0;
+  P.tmin = 0.0f;
+  float dx = 0.0f, dy = 0.0f, dz = 0.0f, tmax = 0.0f;
+  uint32_t best = kMiss;
+  float bt = 0.0f, bu = 0.0f;
+  int node = -1, top = -1, sp = 0;  // the walk: its node, the stack's top entry and the entries below it
+  int *const sh = &s_stack[0][threadIdx.x];
+  int over[kUserDepth - kUserAnyShared];
+  auto test = [&](uint32_t slot) {
+    Ray Q;
+    float nx, ny, nz, unused;
+    up2(P.nxy, nx, ny);
+    up2(P.nzz, nz, unused);
+    Q.ox = -nx;
+    Q.oy = -ny;
+    Q.oz = -nz;
+    Q.tmin = P.tmin;
+    Q.dx = dx;
+    Q.dy = dy;
+    Q.dz = dz;
+    Q.tmax = tmax;
+    const uint32_t id = __ldg(A.ids + slot);
+    float t, u;
+    if (A.prims.hit(Q, id, A.exit_test, t, u) && (best == kMiss || t < bt || (t == bt && id < best))) {
+      best = id;
+      bt = t;
+      bu = u;
+    }
+  };
+  while (true) {
+    if (warp_take(active, drained, A.lanes, kUserRefill, A.nrays, A.counter, r)) {
+      Ray R;
+      ray_setup(__ldg(A.rays + 2 * r), __ldg(A.rays + 2 * r + 1), R);
+      active = true;
+      P = ray_pairs(R);
+      dx = R.dx;
+      dy = R.dy;
+      dz = R.dz;
+      bt = tmax = R.tmax;
+      best = kMiss;
+      node = bt == bt ? 0 : -1;  // no box lies in a range that ends in NaN
+      top = -1;
+      sp = 0;
+      if (A.n == 1) {
+        float tn;
+        if (ray_box(R, A.root_box[0], A.root_box[1], A.root_box[2], A.root_box[3], A.root_box[4], A.root_box[5], bt,
+                    tn))
+          test(0);
+        node = -1;
+      }
+    }
+    if (!__any_sync(FULL_MASK, active)) {
+      if (drained) break;
+      continue;
+    }
+#pragma unroll 1
+    for (int step = 0; step < kUserAnySteps; ++step) {
+      if (node >= 0) {
+        const Bvh2Node *nd = A.bvh + node;
+        const ChildPairs c0 = load_child<V8>(&nd->c[0]), c1 = load_child<V8>(&nd->c[1]);
+        float t0, t1;
+        const bool h0 = child_hit(c0, P, bt, t0), h1 = child_hit(c1, P, bt, t1);
+        if (h0 && c0.ref < 0) test((uint32_t)~c0.ref);
+        if (h1 && c1.ref < 0 && t1 <= bt) test((uint32_t)~c1.ref);
+        const bool in0 = h0 && c0.ref >= 0, in1 = h1 && c1.ref >= 0;
+        const bool first = in0 && !(in1 && t1 < t0);  // the nearer child, child 0 on ties
+        if (best != kMiss) {
+          node = -1;
+        } else if (in0 || in1) {
+          if (in0 && in1) {
+            if (sp < kUserAnyShared) sh[sp * kUserThreads] = top;
+            else if (sp < kUserDepth) over[sp - kUserAnyShared] = top;
+            ++sp;
+            top = first ? c1.ref : c0.ref;
+          }
+          node = first ? c0.ref : c1.ref;
+          if (sp > kUserDepth) {
+            atomicCAS(A.err, 0u, 5u);  // traversal stack overflow
+            node = -1;
+          }
+        } else {
+          node = top;
+          --sp;
+          top = sp < 0 ? -1 : (sp < kUserAnyShared ? sh[sp * kUserThreads] : over[sp - kUserAnyShared]);
+        }
+      }
+    }
+    if (active && node < 0) {
+      Hit h;
+      h.prim = best;
+      h.t = best == kMiss ? __int_as_float(0x7f800000) : bt;
+      A.hits[r] = h;
+      if (A.hit_u) A.hit_u[r] = best == kMiss ? 0.0f : bu;
+      active = false;
+    }
+  }
 }
 
 // The primitive tests of pool_walk (few rays): the ray's direction, and u of
@@ -576,7 +673,7 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolCtas) k_user_pool(const Use
     if (mine) user_hit(A, r, S.best[lane], s_u[w][lane], s_odd[w][lane]);
     __syncwarp();
   }
-  if (lane < kPoolRays) user_odds(A, s_odd[w][lane], false);
+  if (lane < kPoolRays) user_odds(A, s_odd[w][lane]);
 }
 
 }  // namespace gprtcu
@@ -603,17 +700,20 @@ gprtcuStatus trace_user(const gprtcuLbvh *bvh, PRIMS prims, const float *rays, u
   ScratchHeader *hdr = (ScratchHeader *)scratch;
   unsigned long long *counter = reinterpret_cast<unsigned long long *>(&hdr->ticket[0]);
   GPRTCU_TRY(cudaMemsetAsync(scratch, 0, sizeof(ScratchHeader), stream));
-  const RayGrid g = ray_grid(nrays, kUserCtas, kUserWarps);
+  const bool v8 = ((uintptr_t)bvh->bvh2 & 31) == 0;
+  // The pool while it is the faster form: 12/6 chunks per warp, 113,664 rays
+  // on 148 SMs, and 16/6, 151,552 rays, for up to 100,000 primitives.  150,001
+  // rays, plain walk / pool / lane per ray: 10,001 spheres 144 / 143 / 153 us,
+  // 50,001 269 / 250 / 272, 200,001 400 / 409 / 378; 10,001 swept spheres 77 / 81 /
+  // 85, 50,001 186 / 172 / 187, 1,000,001 514 / 519 / 474.
+  const RayGrid few = any ? RayGrid{0, 0} : pool_grid(nrays, 12);
+  const RayGrid g = few.lanes ? few : ray_grid(nrays, any ? kUserAnyCtas : kUserCtas, kUserWarps);
   UserArgs<PRIMS> a{(const Bvh2Node *)bvh->bvh2, bvh->ids, bvh->numPrims, bvh->rootBox, prims, exit_test != 0,
                     (const float4 *)rays, nrays, g.lanes, (Hit *)hits, u, counter, &hdr->status};
-  auto launch = [&](auto kernel) { kernel<<<g.ctas, kUserThreads, 0, stream>>>(a); };
-  const bool v8 = ((uintptr_t)bvh->bvh2 & 31) == 0;
-  if (const RayGrid few = pool_grid(nrays); !any && few.lanes) {
-    a.lanes = few.lanes;
-    if (v8) k_user_pool<PRIMS, true><<<few.ctas, kPoolThreads, 0, stream>>>(a);
-    else k_user_pool<PRIMS, false><<<few.ctas, kPoolThreads, 0, stream>>>(a);
-  } else if (any) v8 ? launch(k_trace_user<PRIMS, true, true>) : launch(k_trace_user<PRIMS, true, false>);
-  else v8 ? launch(k_trace_user<PRIMS, false, true>) : launch(k_trace_user<PRIMS, false, false>);
+  auto launch = [&](auto kernel, int threads) { kernel<<<g.ctas, threads, 0, stream>>>(a); };
+  if (any) v8 ? launch(k_user_any<PRIMS, true>, kUserThreads) : launch(k_user_any<PRIMS, false>, kUserThreads);
+  else if (few.lanes) v8 ? launch(k_user_pool<PRIMS, true>, kPoolThreads) : launch(k_user_pool<PRIMS, false>, kPoolThreads);
+  else v8 ? launch(k_user_closest<PRIMS, true>, kUserThreads) : launch(k_user_closest<PRIMS, false>, kUserThreads);
   GPRTCU_TRY(cudaGetLastError());
   return GPRTCU_OK;
 }

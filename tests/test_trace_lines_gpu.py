@@ -1,0 +1,92 @@
+"""The ray counts at which a traversal changes its form: the same hits on both
+sides of each line, and no step in time at the line of the shared-visit form
+that goes up as more rays come."""
+import numpy as np
+import pytest
+
+import oracle
+from gprt_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def _line(sixths):
+    """The largest ray count of the shared-visit form: that many sixths of 16
+    rays for each of 12 x 2 warps per SM."""
+    return _sms() * 12 * 2 * 16 * sixths // 6
+
+
+def _bits(h):
+    return h.cpu().numpy().view(np.uint32)
+
+
+@pytest.mark.parametrize("n,sixths", [(2047, 6), (2048, 9)])
+def test_triangle_line(cuda, n, sixths):
+    import torch
+    from gprt_b200 import api
+    m = _line(sixths)
+    pos, tri = scenes.soup(n, seed=n, sigma=0.03)
+    rays_h = scenes.rays(m + 1, seed=n)
+    rays = torch.from_numpy(rays_h).cuda()
+    b = api.lbvh_build_triangles(torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda())
+    below, above = _bits(api.trace(b, rays[:m])), _bits(api.trace(b, rays))
+    assert np.array_equal(below, above[:m])
+    exp = oracle.trace_lbvh(pos, tri, oracle.lbvh_build_tri(pos, tri), rays_h[-3000:])
+    assert np.array_equal(above[-3000:, 0], exp["prim"])
+
+
+@pytest.mark.parametrize("n,sixths", [(100000, 16), (100001, 12)])
+@pytest.mark.parametrize("kind", ["spheres", "lss"])
+def test_prim_line(cuda, n, sixths, kind):
+    import torch
+    from gprt_b200 import api
+    m = _line(sixths)
+    rng = np.random.default_rng(n)
+    v = np.concatenate([rng.random((n + 1, 3)), rng.uniform(0.001, 0.004, (n + 1, 1))], 1).astype(np.float32)
+    v[1::2, :3] = v[:-1:2, :3][:len(v[1::2])] + rng.normal(0, 0.004, (len(v[1::2]), 3)).astype(np.float32)
+    idx = np.stack([np.arange(n) & ~1, (np.arange(n) & ~1) + 1], 1).astype(np.uint32) % (n + 1)
+    rays_h = scenes.rays(m + 1, seed=n)
+    rays, vt, it = torch.from_numpy(rays_h).cuda(), torch.from_numpy(v).cuda(), torch.from_numpy(idx.view(np.int32)).cuda()
+    if kind == "spheres":
+        b = api.lbvh_build_boxes(api.sphere_bounds(vt[:n]))
+        run = lambda r, u: api.trace_spheres(b, vt[:n], r, u=u)
+    else:
+        b = api.lbvh_build_boxes(api.lss_bounds(vt, it))
+        run = lambda r, u: api.trace_lss(b, vt, it, r, u=u)
+    u = [torch.zeros(m + 1, device="cuda") for _ in range(2)]
+    below, above = _bits(run(rays[:m], u[0])), _bits(run(rays, u[1]))
+    assert np.array_equal(below, above[:m])
+    assert torch.equal(u[0][:m].view(torch.int32), u[1][:m].view(torch.int32))
+    e = oracle.trace_user_brute(0 if kind == "spheres" else 1, v[:n] if kind == "spheres" else v, rays_h[-300:],
+                                *(() if kind == "spheres" else (idx,)))
+    assert np.array_equal(above[-300:, 0], e["prim"])
+
+
+@pytest.mark.parametrize("n", [1, 2, 5000])
+def test_any_hit_whatever_the_rays(cuda, n):
+    """An any-hit call reports the first hit of the near-first walk, so the
+    same one however many rays the call has and however they share warps."""
+    import torch
+    from gprt_b200 import api
+    pos, tri = scenes.soup(n, seed=n + 3, sigma=0.1)
+    rays = torch.from_numpy(scenes.rays(200003, seed=n)).cuda()
+    b = api.lbvh_build_triangles(torch.from_numpy(pos).cuda(), torch.from_numpy(tri.view(np.int32)).cuda())
+    sph = torch.from_numpy(np.concatenate([np.random.default_rng(n).random((n + 1, 3)), np.full((n + 1, 1), 0.04)],
+                                          1).astype(np.float32)).cuda()
+    idx = torch.stack([torch.arange(n), torch.arange(n) + 1], 1).int().cuda()
+    bs, bl = api.lbvh_build_boxes(api.sphere_bounds(sph[:n])), api.lbvh_build_boxes(api.lss_bounds(sph, idx))
+    runs = [lambda r, u: api.trace(b, r, anyhit=True),
+            lambda r, u: api.trace_spheres(bs, sph[:n], r, u=u, anyhit=True),
+            lambda r, u: api.trace_lss(bl, sph, idx, r, u=u, anyhit=True)]
+    for run in runs:
+        u = torch.zeros(200003, device="cuda")
+        full = _bits(run(rays, u)).copy()
+        for m in (1, 33, 700, 4099, 30011, 56001):
+            v = torch.zeros(m, device="cuda")
+            assert np.array_equal(_bits(run(rays[:m], v)), full[:m])
+            assert torch.equal(v.view(torch.int32), u[:m].view(torch.int32))
