@@ -207,11 +207,11 @@ template <typename PRIMS> struct UserArgs {
 
 constexpr int kUserThreads = 128;
 constexpr int kUserWarps = kUserThreads / 32;
-constexpr int kUserCtas = 8;
+constexpr int kUserCtas = 7;
 constexpr int kUserShared = 12;  // stack entries in shared memory
 constexpr int kUserDepth = 64;
 constexpr int kUserRefill = 8;
-constexpr int kUserSteps = 10;
+constexpr int kUserSteps = 14;
 constexpr int kUserFlush = 12;
 constexpr int kUserQueue = 96;  // a step queues at most 64
 
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kUserThreads, kUserCtas) k_user_closest(const 
     const bool done = W.node == kWalkEnd;
     const unsigned waiting = __ballot_sync(FULL_MASK, done && active && pending);
     const unsigned running = __ballot_sync(FULL_MASK, active && !done);
-    if (nq >= kUserFlush ||
+    if (nq >= kUserFlush || (drained && nq >= __popc(running)) ||
         (waiting && (!running || A.lanes - __popc(running) >= kUserRefill)))
       flush();
     if (active && done && !pending) {
@@ -706,7 +706,7 @@ gprtcuStatus trace_user(const gprtcuLbvh *bvh, PRIMS prims, const float *rays, u
   // rays, plain walk / pool / lane per ray: 10,001 spheres 144 / 143 / 153 us,
   // 50,001 269 / 250 / 272, 200,001 400 / 409 / 378; 10,001 swept spheres 77 / 81 /
   // 85, 50,001 186 / 172 / 187, 1,000,001 514 / 519 / 474.
-  const RayGrid few = any ? RayGrid{0, 0} : pool_grid(nrays, 12);
+  const RayGrid few = any ? RayGrid{0, 0} : pool_grid(nrays, bvh->numPrims <= 100000 ? 16 : 12);
   const RayGrid g = few.lanes ? few : ray_grid(nrays, any ? kUserAnyCtas : kUserCtas, kUserWarps);
   UserArgs<PRIMS> a{(const Bvh2Node *)bvh->bvh2, bvh->ids, bvh->numPrims, bvh->rootBox, prims, exit_test != 0,
                     (const float4 *)rays, nrays, g.lanes, (Hit *)hits, u, counter, &hdr->status};

@@ -90,3 +90,33 @@ def test_any_hit_whatever_the_rays(cuda, n):
             v = torch.zeros(m, device="cuda")
             assert np.array_equal(_bits(run(rays[:m], v)), full[:m])
             assert torch.equal(v.view(torch.int32), u[:m].view(torch.int32))
+
+
+def test_no_step_at_the_line(cuda):
+    """Spheres, around twice 16 rays for every warp that fits, where the lane
+    per ray takes over: a call with a few more rays does not take clearly
+    longer, nor does one with fewer."""
+    import torch
+    from gprt_b200 import api
+    n, m, slack = 1_000_001, _line(12), 1.2
+    a, b = int(m * 0.994), int(m * 1.012)
+    rays = api.gen_rays(b, seed=5)
+    s = torch.rand((n, 4), generator=torch.Generator("cuda").manual_seed(1), device="cuda")
+    s[:, 3].mul_(0.0015).add_(0.0005)
+    t = api.lbvh_build_boxes(api.sphere_bounds(s))
+    hits, scr = torch.empty((b, 2), dtype=torch.int32, device="cuda"), api.scratch(256)
+
+    def us(r):
+        times = []
+        for _ in range(9):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            for _ in range(10):
+                api.trace_spheres(t, s, r, hits=hits[:r.shape[0]], scr=scr)
+            e[1].record()
+            e[1].synchronize()
+            times.append(1e2 * e[0].elapsed_time(e[1]))
+        return sorted(times[2:])[3]
+
+    below, above = us(rays[:a]), us(rays)
+    assert above < slack * below and below < slack * above, (below, above)
