@@ -643,6 +643,21 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolCtas) k_user_pool(const Use
   PoolShared &S = s_pool[w];
   const PoolPrims<PRIMS> prims{A, s_dir[w], s_u[w]};
   if (lane < kPoolRays) s_odd[w][lane] = odd_link(kOddEnd);
+  // The shared visits meet the tests in another order than user_odd, and can
+  // pass by a primitive that would give a distance that is no number: rays
+  // for which one could, go there at once.  With m the larger of the distances
+  // from zero of the ray's origin and the scene's farthest corner, all that
+  // the last test of lss_intersect forms is below 100 m^2 |d|^2, 100 m^2 and 4 m
+  // / |d|, and the first has no hit unless its own t is a number.  (A
+  // primitive with a NaN coordinate is in no box but its own, so the scene's
+  // does not show it: whether such a one is met before a nearer hit is left
+  // open.)
+  float corner = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float c = fmaxf(fabsf(__ldg(A.root_box + k)), fabsf(__ldg(A.root_box + 3 + k)));
+    corner += c * c;
+  }
   while (true) {
     unsigned long long first = 0;
     if (lane == 0) first = atomicAdd(A.counter, (unsigned long long)A.lanes);
@@ -655,10 +670,9 @@ __global__ void __launch_bounds__(kPoolThreads, kPoolCtas) k_user_pool(const Use
       Ray R;
       ray_setup(__ldg(A.rays + 2 * r), __ldg(A.rays + 2 * r + 1), R);
       pool_ray(S, lane, R, 0u, 0u);
-      // the walk below meets the tests in another order than user_odd: rays
-      // that are likely odd go there at once
-      const float oo = R.ox * R.ox + R.oy * R.oy + R.oz * R.oz, dd = R.dx * R.dx + R.dy * R.dy + R.dz * R.dz;
-      if (!(oo < 1e30f && dd < 1e30f && dd > 1e-30f)) S.best[lane] = kOddKey;
+      const float mm = R.ox * R.ox + R.oy * R.oy + R.oz * R.oz + corner;
+      const float dd = R.dx * R.dx + R.dy * R.dy + R.dz * R.dz;
+      if (!(mm * fmaxf(dd, 1.0f) < 1e30f && dd < 1e30f && dd > 1e-30f)) S.best[lane] = kOddKey;
       s_dir[w][lane] = make_float4(R.dx, R.dy, R.dz, 0.0f);
       if (A.n == 1) {
         float tn;

@@ -350,3 +350,39 @@ def test_ranges_behind_the_origin(cuda, m):
     got = api.hits_numpy(api.trace_spheres(api.lbvh_build_boxes(api.sphere_bounds(s)), s, r))
     e = oracle.trace_user_brute(0, sph, rays)
     assert np.array_equal(got["prim"], e["prim"]) and (e["prim"] != 0xFFFFFFFF).sum() > m // 10
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e14])
+def test_prims_odd_prims(cuda, scale):
+    """Swept spheres that reach so far that squares overflow and a test's
+    distance is no number (or, at 1e14 with directions as long, where every
+    test's is).  Such a hit counts if it is the ray's first in near-first
+    order: one lies behind ordinary ones but in the nearer half of the tree.
+    The same hits however many rays the call has."""
+    import torch
+    from gprt_b200 import api
+    few, many = 100003, 300007
+    rng = np.random.default_rng(11)
+    far = 1e20 if scale == 1.0 else 60.0
+    v = np.zeros((522, 4))
+    v[0::2, 0] = 10.0 + 0.1 * np.arange(261)  # 256 that reach far, all from x = 10 on
+    v[1::2, 0] = far
+    v[0, 0], v[:2, 1] = 1.0, 50.0  # the first of them starts nearer, off to the side
+    v[512:520] = np.repeat([[5.0, 0.0, 0.0, 0.0], [5.1, 0.0, 0.0, 0.0], [5.2, 0.0, 0.0, 0.0], [5.3, 0.0, 0.0, 0.0]], 2, 0)
+    v[513:520:2, 0] += 0.2
+    v[520:, :3] = [[far, far, far], [far, -far, -far]]  # the scene as wide as it is long: the first one in their cell
+    v[:, 3] = 1.0
+    rays = np.zeros((many, 8))
+    rays[:, 1:3] = rng.uniform(-0.05, 0.05, (many, 2))
+    rays[:, 4] = 1.0
+    rays[:, 7] = np.inf
+    v, rays[:, :3], rays[:, 4:7] = v * scale, rays[:, :3] * scale, rays[:, 4:7] * scale
+    idx = np.arange(522, dtype=np.int32).reshape(261, 2)
+    vt, it = torch.from_numpy(v.astype(np.float32)).cuda(), torch.from_numpy(idx).cuda()
+    r = torch.from_numpy(rays.astype(np.float32)).cuda()
+    b = api.lbvh_build_boxes(api.lss_bounds(vt, it))
+    u = torch.zeros(many, device="cuda"), torch.zeros(few, device="cuda")
+    full, part = api.trace_lss(b, vt, it, r, u=u[0]), api.trace_lss(b, vt, it, r[:few].contiguous(), u=u[1])
+    assert int(torch.isnan(full[:few, 1].view(torch.float32)).sum()) > few // 2
+    assert torch.equal(full[:few], part)
+    assert torch.equal(u[0][:few].view(torch.int32), u[1].view(torch.int32))
