@@ -28,6 +28,8 @@
 
 #include <type_traits>
 
+uint32_t gprtcu_spin_budget(void);
+
 namespace gprtcu {
 
 struct __align__(16) WideNode {
@@ -61,8 +63,10 @@ struct WorkItem {
 // Collapse counters: the current level's items are queue[LO, HI); TAIL is
 // the next free queue slot (= the number of wide nodes so far: a wide node's
 // index is its queue slot), LEAF the next free wide leaf slot, TICKET the
-// level kernel's CTA done-counter.
-enum { C_LO = 0, C_HI = 1, C_TAIL = 2, C_LEAF = 3, C_TICKET = 4 };
+// level kernel's CTA done-counter, EPOCH and NEXT (polled, so in a line of
+// their own) the levels that the last launch has finished and TAIL after the
+// latest of them.
+enum { C_LO = 0, C_HI = 1, C_TAIL = 2, C_LEAF = 3, C_TICKET = 4, C_EPOCH = 32, C_NEXT = 33 };
 
 // Levels a collapse runs: a binary node splits its keys at the highest
 // differing bit of (30-bit code, 30-bit index), so binary and therefore wide
@@ -114,10 +118,13 @@ __global__ void k_wide_init(const uint32_t *tri_off, uint32_t meshes, uint32_t n
 // queue slots and leaf slots with one atomic add each (prefix sums across
 // the lanes); the last CTA to finish advances [LO, HI) to the items just
 // appended.  These levels run as successive launches, so nothing waits on
-// another thread's progress.  CLUSTER is the form for levels with few items
-// (the first ones of a mesh and the last): one thread-block cluster goes from
-// level to level by itself, a hardware barrier between them, while a level
-// has at most `most` items.  The eight candidate children stay in registers
+// another thread's progress.  kWideClusterForm is the form for levels with few
+// items (the first ones of a mesh and the last): one thread-block cluster goes
+// from level to level by itself, a hardware barrier between them, while a level
+// has at most `most` items.  kWideRestForm takes whatever levels are left: all
+// its CTAs are on the GPU at once (a cooperative launch) and wait for one
+// another after each level, `most` polls at most, after which the call's
+// status is GPRTCU_ERR_TIMEOUT.  The eight candidate children stay in registers
 // (unrolled loops, predicated updates) and quantising multiplies by the exact
 // power of two 2^-e instead of dividing by 2^e: on 67M triangles in 16,384
 // meshes the collapse went from 10.96 ms (local-memory arrays, FP64
@@ -127,20 +134,21 @@ __global__ void k_wide_init(const uint32_t *tri_off, uint32_t meshes, uint32_t n
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
-template <bool CLUSTER>
-__global__ void __launch_bounds__(128, CLUSTER ? 1 : 7) k_wide_level(const Bvh2Node *bvh2, const float4 *leaf_tris,
+enum { kWideLevelForm, kWideClusterForm, kWideRestForm };
+template <int FORM>
+__global__ void __launch_bounds__(128, FORM == kWideClusterForm ? 1 : 7) k_wide_level(const Bvh2Node *bvh2, const float4 *leaf_tris,
                                                     const uint32_t *tri_off, WideNode *wnodes, float4 *wleaf,
                                                     WorkItem *queue, uint32_t *counters, uint32_t most) {
   uint32_t lo = counters[C_LO], hi = counters[C_HI];
   // an empty level appends nothing, so the next window equals this one: the
   // launch leaves the counters as they are
-  if (lo == hi || (CLUSTER && hi - lo > most)) return;
+  if (lo == hi || (FORM == kWideClusterForm && hi - lo > most)) return;
   const int lane = threadIdx.x & 31;
   // candidate child boxes, thread-private: [coordinate][slot][thread]
   __shared__ float s_box[6][8][128];
 #define CBOX(c, k) s_box[(k)][(c)][threadIdx.x]
   const uint32_t stride = gridDim.x * blockDim.x;
-  for (int level = 0; level < (CLUSTER ? kWideMaxLevels : 1); ++level) {
+  for (int level = 0; level < (FORM == kWideLevelForm ? 1 : kWideMaxLevels); ++level) {
     const uint32_t total = hi - lo;
     for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < total; i0 += stride) {
       const uint32_t idx = lo + i0 + lane;
@@ -302,7 +310,37 @@ __global__ void __launch_bounds__(128, CLUSTER ? 1 : 7) k_wide_level(const Bvh2N
       op[wide_word(idx, 3)] = make_uint4(qlo_w[2][0], qlo_w[2][1], qhi_w[0][0], qhi_w[0][1]);
       op[wide_word(idx, 4)] = make_uint4(qhi_w[1][0], qhi_w[1][1], qhi_w[2][0], qhi_w[2][1]);
     }
-    if constexpr (CLUSTER) {
+    if constexpr (FORM == kWideRestForm) {
+      // the last CTA to finish the level tells the others how many items the
+      // next one has
+      __shared__ uint32_t s_next;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        __threadfence();
+        uint32_t next = 0;
+        if (atomicAdd(&counters[C_TICKET], 1u) == gridDim.x - 1) {
+          __threadfence();
+          next = ld_relaxed_u32(&counters[C_TAIL]);
+          st_relaxed_u32(&counters[C_TICKET], 0u);
+          st_relaxed_u32(&counters[C_NEXT], next);
+          __threadfence();
+          st_relaxed_u32(&counters[C_EPOCH], (uint32_t)level + 1u);
+        } else {
+          bool ok = false;
+          for (uint32_t i = 0; !ok && i <= most; ++i) ok = ld_acquire_u32(&counters[C_EPOCH]) > (uint32_t)level;
+          if (ok) next = ld_relaxed_u32(&counters[C_NEXT]);
+          else record_error(reinterpret_cast<ScratchHeader *>(reinterpret_cast<char *>(counters) - sizeof(ScratchHeader)),
+                            GPRTCU_ERR_TIMEOUT);
+        }
+        s_next = next;
+      }
+      __syncthreads();
+      const uint32_t tail = s_next;
+      if (tail <= hi) break;  // no items left (or the wait ran out)
+      lo = hi;
+      hi = tail;
+    }
+    if constexpr (FORM == kWideClusterForm) {
       cluster_sync();  // the next level's items are written
       const uint32_t tail = ld_relaxed_u32(&counters[C_TAIL]);
       cluster_sync();  // and everyone knows how many before they append to them
@@ -312,13 +350,13 @@ __global__ void __launch_bounds__(128, CLUSTER ? 1 : 7) k_wide_level(const Bvh2N
     }
   }
 #undef CBOX
-  if constexpr (CLUSTER) {
+  if constexpr (FORM == kWideClusterForm) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       counters[C_LO] = lo;
       counters[C_HI] = hi;
     }
-    return;
   }
+  if constexpr (FORM != kWideLevelForm) return;
   // the last CTA to finish moves the level window to the appended items
   __shared__ bool s_last;
   __syncthreads();
@@ -916,30 +954,35 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuWideBuild(const gprtcuLbvh *binary, con
   int level_ctas = level_ctas_cache.load(std::memory_order_relaxed);
   if (!level_ctas) {
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wide_level<false>, 128, 0) != cudaSuccess || occ < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wide_level<kWideRestForm>, 128, 0) != cudaSuccess || occ < 1)
       occ = 1;
     level_ctas = occ;
     level_ctas_cache.store(occ, std::memory_order_relaxed);
   }
   const int grid = gprtcu_num_sms() * level_ctas;
-  auto launch = [&](auto kernel, int ctas, int cluster, uint32_t most) -> cudaError_t {
+  auto launch = [&](auto kernel, int ctas, cudaLaunchAttribute at, uint32_t most) -> cudaError_t {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(128);
     cfg.stream = stream;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = cluster;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, (const Bvh2Node *)binary->bvh2, (const float4 *)binary->leafTris, toff,
                               (WideNode *)out->nodes, (float4 *)out->leafTris, queue, counters, most);
   };
-  auto few = [&](uint32_t most) { return launch(k_wide_level<true>, kWideCluster, kWideCluster, most); };
+  cudaLaunchAttribute cluster = {}, rest = {};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  rest.id = cudaLaunchAttributeCooperative;
+  rest.val.cooperative = 1;
+  auto few = [&](uint32_t most) {
+    cluster.val.clusterDim.x = kWideCluster;
+    return launch(k_wide_level<kWideClusterForm>, kWideCluster, cluster, most);
+  };
   auto levels = [&](int count) -> cudaError_t {
+    cluster.val.clusterDim.x = 1;
     for (int i = 0; i < count; ++i) {
-      const cudaError_t e = launch(k_wide_level<false>, grid, 1, 0u);
+      const cudaError_t e = launch(k_wide_level<kWideLevelForm>, grid, cluster, 0u);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -950,24 +993,27 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuWideBuild(const gprtcuLbvh *binary, con
   // So: the cluster takes the first levels, up to kWideFew items; as many
   // whole-GPU levels follow as scenes of n triangles have needed (8 to 13
   // levels in all for 20,001 to 4.2 M of them, 10 for a batch of 67 M); the
-  // cluster goes on while at most kWideMore items are left, which is
-  // usually the end; a few whole-GPU levels are for a tree that widens again
-  // that late, and the cluster ends what is left.  Up to 100,000 triangles the
-  // cluster alone is no slower than the 62 launches were.
-  //   1,501 triangles 0.36 -> 0.06 ms; 20,001 0.31 -> 0.08; 262,144 0.33 ->
-  //   0.12; 1 M 0.42 -> 0.21; 4.2 M 0.75 -> 0.55; 67 M in 4,096 meshes 2.97 ->
-  //   2.75 ms.  The cluster alone: 0.06, 0.10, 0.58, 3.8, 18 ms.
+  // cluster goes on while at most kWideMore items are left, which is usually
+  // the end; and one launch takes what then is left of a tree that stays wide,
+  // or widens again, that late.  Up to 100,000 triangles the cluster alone is
+  // no slower than the 62 launches were.
+  //   1,501 triangles 0.36 -> 0.06 ms; 20,001 0.31 -> 0.08; 150,001 0.33 ->
+  //   0.10; 1 M 0.41 -> 0.19; 4.2 M 0.64 -> 0.43; 67 M in 4,096 meshes 2.97 ->
+  //   2.75 ms.  In meshes graded towards a point most levels come late: 1 M /
+  //   4.2 M triangles over 25 octaves of distance 0.64 / 0.84 ms with 62
+  //   launches, 2.8 / 10.7 with the cluster to end them, 0.50 / 0.69 so.
   int lg = 0;
   while (lg < 32 && (1ull << lg) < n) ++lg;
   if (n > 8192) {
     GPRTCU_TRY(few(kWideFew));
     GPRTCU_TRY(levels(lg > 16 ? lg - 14 : 2));
-    if (n > 100000) {
-      GPRTCU_TRY(few(kWideMore));
-      GPRTCU_TRY(levels(4));
-    }
   }
-  GPRTCU_TRY(few(UINT32_MAX));
+  if (n > 100000) {
+    GPRTCU_TRY(few(kWideMore));
+    GPRTCU_TRY(launch(k_wide_level<kWideRestForm>, grid, rest, gprtcu_spin_budget()));
+  } else {
+    GPRTCU_TRY(few(UINT32_MAX));
+  }
   if (out->numNodes) GPRTCU_TRY(cudaMemcpyAsync(out->numNodes, counters + C_TAIL, 4, cudaMemcpyDeviceToDevice, stream));
   return GPRTCU_OK;
 }
