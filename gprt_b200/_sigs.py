@@ -66,6 +66,7 @@ SIGNATURES = {
     "gprtcuDebugSortPrefetch": ([i32], None),
     "gprtcuDebugRefitSkipLeaf": ([i64], st),
     "gprtcuDebugScanImpl": ([i32], None),
+    "gprtcuDebugMaxCluster": ([i32], None),
 }
 
 

@@ -217,3 +217,8 @@ __device__ __forceinline__ uint32_t mbar_budget_of(uint32_t lookback_budget) {
 
 // Number of SMs of the current device (cached per device id).
 int gprtcu_num_sms();
+// Largest thread-block cluster, a power of two up to 16, that the current
+// device can run (cached per device id): 16 on a whole B200, less where the
+// GPU is partitioned into parts whose processor groups are small.  Calls with
+// a form that is one cluster ask first and take their general form otherwise.
+int gprtcu_max_cluster();

@@ -1062,6 +1062,40 @@ static void launch_reg_scan(const uint32_t *in, uint32_t *out, uint64_t n, int i
 #undef GPRTCU_SCAN_LAUNCH
 }
 
+static std::atomic<int> g_max_cluster{0};
+extern "C" GPRTCU_API void gprtcuDebugMaxCluster(int ctas) { g_max_cluster.store(ctas, std::memory_order_relaxed); }
+
+// Asked of the occupancy calculator with the partition kernel, whose CTAs are
+// the largest of those that run in clusters (256 threads, 33 KB).
+int gprtcu_max_cluster() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  int v = cached[dev].load(std::memory_order_relaxed);
+  if (v == 0) {
+    const auto kernel = k_partition_i32<true, true, true>;
+    const bool wide =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    for (v = wide ? 16 : 8; v > 1; v >>= 1) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(v);
+      cfg.blockDim = dim3(SCAN_THREADS);
+      cudaLaunchAttribute at = {};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = v;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit > 0) break;
+    }
+    cudaGetLastError();
+    cached[dev].store(v, std::memory_order_relaxed);
+  }
+  const int most = g_max_cluster.load(std::memory_order_relaxed);
+  return most > 0 && most < v ? most : v;
+}
+
 // Launches `kernel` as one cluster of the next power of two of `tiles` CTAs
 // (those past the last tile only take part in the barriers).
 template <typename... P, typename... A>
@@ -1085,6 +1119,11 @@ static cudaError_t launch_cluster(void (*kernel)(P...), uint64_t tiles, int thre
   return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
 }
 
+// Whether `tiles` run as one cluster here.
+static bool cluster_tiles(uint64_t tiles) {
+  return tiles <= kClusterTiles && tiles <= (uint64_t)gprtcu_max_cluster();
+}
+
 static gprtcuStatus scan_launch(const uint32_t *in, uint32_t *out, uint64_t n, int inclusive, uint32_t *d_total,
                                 void *scratch, size_t scratch_bytes, cudaStream_t stream) {
   if (n > kScanMaxN) return GPRTCU_ERR_TOO_LARGE;
@@ -1105,7 +1144,7 @@ static gprtcuStatus scan_launch(const uint32_t *in, uint32_t *out, uint64_t n, i
   const uint64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
   if (scratch_bytes < sizeof(ScratchHeader) + tiles * sizeof(uint64_t)) return GPRTCU_ERR_SCRATCH_TOO_SMALL;
   // few tiles: one cluster (not with a test hook set: those are of the others)
-  if (n > 0 && tiles <= kClusterTiles && g_scan_impl == 0 && g_skip_tile < 0) {
+  if (n > 0 && cluster_tiles(tiles) && g_scan_impl == 0 && g_skip_tile < 0) {
 #define GPRTCU_SCAN_CLUSTER(M, V, N)                                                                          \
   GPRTCU_TRY(launch_cluster(k_scan_u32<M, V, N, SCAN_THREADS, SCAN_VECS, 32, true>, tiles, SCAN_THREADS, stream, in, \
                             out, n, tiles, hdr, status, d_total, g_spin_budget, g_skip_tile))
@@ -1172,7 +1211,7 @@ static gprtcuStatus partition_launch(const int32_t *in, int32_t *out, uint64_t n
   uint64_t *status = (uint64_t *)((char *)scratch + sizeof(ScratchHeader));
   uint64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
   const bool vec = ((uintptr_t)in & 15) == 0;
-  if (n > 0 && tiles <= kClusterTiles && g_scan_impl == 0) {
+  if (n > 0 && cluster_tiles(tiles) && g_scan_impl == 0) {
 #define GPRTCU_PART_CLUSTER(P, V)                                                                         \
   GPRTCU_TRY(launch_cluster(k_partition_i32<P, V, true>, tiles, SCAN_THREADS, stream, in, out, n, tiles, \
                             select_positive, hdr, status, d_count, g_spin_budget))

@@ -1004,13 +1004,13 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuWideBuild(const gprtcuLbvh *binary, con
   //   launches, 2.8 / 10.7 with the cluster to end them, 0.50 / 0.69 so.
   int lg = 0;
   while (lg < 32 && (1ull << lg) < n) ++lg;
-  if (n > 8192) {
+  if (gprtcu_max_cluster() < kWideCluster) {
+    GPRTCU_TRY(launch(k_wide_level<kWideRestForm>, grid, rest, gprtcu_spin_budget()));
+  } else if (n > 8192) {
     GPRTCU_TRY(few(kWideFew));
     GPRTCU_TRY(levels(lg > 16 ? lg - 14 : 2));
-  }
-  if (n > 100000) {
-    GPRTCU_TRY(few(kWideMore));
-    GPRTCU_TRY(launch(k_wide_level<kWideRestForm>, grid, rest, gprtcu_spin_budget()));
+    GPRTCU_TRY(few(n > 100000 ? kWideMore : UINT32_MAX));
+    if (n > 100000) GPRTCU_TRY(launch(k_wide_level<kWideRestForm>, grid, rest, gprtcu_spin_budget()));
   } else {
     GPRTCU_TRY(few(UINT32_MAX));
   }

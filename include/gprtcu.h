@@ -496,6 +496,11 @@ GPRTCU_API gprtcuStatus gprtcuDebugRefitSkipLeaf(int64_t slot);
  * 1 = register-staged tile per CTA, 2 = TMA-staged tile per CTA,
  * 3 = persistent re-read kernel (2 and 3 need 16-byte aligned in/out). */
 GPRTCU_API void gprtcuDebugScanImpl(int impl);
+/* The largest thread-block cluster that calls may count on, for tests: as on a
+ * GPU partitioned so that larger ones do not fit (0 restores what the device
+ * has).  Sums, partition and select of few tiles and the collapse then take
+ * the forms without such a cluster; all give the same results. */
+GPRTCU_API void gprtcuDebugMaxCluster(int ctas);
 
 #ifdef __cplusplus
 }
