@@ -16,8 +16,17 @@ from . import GprtcuError, lib
 # resolving the device from Python: 5 of the 9.5 us that a call of a few
 # microseconds of GPU work took on the host (a sum of 99,730 elements: 9.5 ->
 # 6.0 us per call, 4.5 of them on the host).
-def _stream():
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+# Both functions are internal to torch; a torch without one of them gets the
+# documented form.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", None)
+
+if _raw_stream is not None and _raw_device is not None:
+    def _stream():
+        return _raw_stream(_raw_device())
+else:
+    def _stream():
+        return torch.cuda.current_stream().cuda_stream
 
 
 def _ptr(t):
