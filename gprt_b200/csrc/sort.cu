@@ -76,9 +76,13 @@ int grid_index(int rb, int tile, int warps) {
 // a chain of look-backs from tile to tile, so few large tiles beat many small
 // ones as soon as they fill most of the SMs (times of whole sorts in us):
 //   below 2^19 keys 2048-key tiles (2^18 u32 pairs: 57 at 2048, 59 at 4096, 66
-//     at 8192), below 2^20 4096-key ones (2^19 u64/u32 pairs: 100 / 90 / 100);
-//   while 8192-key tiles all fit on the GPU at once (two CTAs per SM, one
-//     where key and payload take 12 bytes or more) 8192 (2^20 u32 pairs: 93 /
+//     at 8192);
+//   from there the smallest tile of which every SM gets at most one, 4096,
+//     6144, then 8192 (u64 pairs of 700,001 keys, 171 / 114 / 86 tiles: 162 /
+//     131 / 131, with 2048 150; of 1,000,001, 245 / 163 / 123 tiles: 154 / 191 /
+//     144; u32 pairs 81 / 65 / 66 and 75 / 75 / 69);
+//   and 8192 on while those tiles all fit on the GPU at once (two CTAs per SM,
+//     one where key and payload take 12 bytes or more; 2^20 u32 pairs: 93 /
 //     83 / 75; 2^21: 133 / 111 / 103; 2^20 u64/u32 pairs 137 / 116 / 111; 2^20
 //     u64 pairs 140 / 124 / 112);
 //   beyond, 6144-key tiles, of which three CTAs share an SM with 32-bit keys
@@ -86,16 +90,24 @@ int grid_index(int rb, int tile, int warps) {
 //     2^28 Zipf pairs 5.76 ms against 5.95 at 8192; 2^26 segmented u64/u32
 //     pairs of 44 bits 3.09 ms against 3.14 at 4096; 10^8 u64 keys 4.56 ms
 //     against 5.00 at 4096), except u32 keys alone 8192 (2^28 Zipf keys 4.66 ms
-//     against 4.81) and u64 pairs 4096 with 16 warps (4.2 M: 349 against 384
-//     with 8 warps) and from 2^23 on 8192 with 16 warps (10^8: 7.13 ms against
-//     7.38 at 4096 and 8.03 at 6144).
+//     against 4.81) and u64 pairs, at 4096 with 16 / 4096 with 8 / 8192 with 16
+//     warps: 6.0 M 655 / 681 / 627 uniform and 418 / 420 / 382 Zipf, 8.0 M 795 /
+//     764 / 827 and 514 / 485 / 496, 9.0 M 879 / 862 / 920 and 570 / 542 / 547,
+//     11.0 M 1,067 / 1,061 / 1,087 and 685 / 661 / 649, 14.0 M 1,353 / 1,365 /
+//     1,365 and 864 / 839 / 807, 10^8 - / 7.38 / 7.13 ms: the first below 7.5 M
+//     (level with the third from 3 M to 5 M), the third from 11.5 M on.
 int default_index(int slot, uint64_t n) {
+  const uint64_t sms = (uint64_t)gprtcu_num_sms();
   if (n < (1ull << 19)) return grid_index(8, 2048, 8);
-  if (n < (1ull << 20)) return grid_index(8, 4096, 8);
+  if (n <= sms * 4096) return grid_index(8, 4096, 8);
+  if (n <= sms * 6144) return grid_index(8, 6144, 8);
   const uint64_t per_sm = slot <= 2 ? 2 : 1;  // 8192-key CTAs that share an SM
-  if (n <= per_sm * (uint64_t)gprtcu_num_sms() * 8192) return grid_index(8, 8192, 8);
+  if (n <= per_sm * sms * 8192) return grid_index(8, 8192, 8);
   if (slot == 0) return grid_index(8, 8192, 8);
-  if (slot == 4) return n < (1ull << 23) ? grid_index(8, 4096, 16) : grid_index(8, 8192, 16);
+  if (slot == 4) {
+    if (n < 7500000) return grid_index(8, 4096, 16);
+    return n < 11500000 ? grid_index(8, 4096, 8) : grid_index(8, 8192, 16);
+  }
   return grid_index(8, 6144, 8);
 }
 
