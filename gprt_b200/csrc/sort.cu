@@ -199,7 +199,9 @@ gprtcuStatus sort_dispatch(int slot, int index, void *keys, void *vals, uint64_t
   a.budget = gprtcu_spin_budget();
   a.skip_tile = g_sort_skip_tile;
   a.pf_tiles = 0;
-  a.use_bulk = ((((uintptr_t)keys) | ((uintptr_t)a.keys_alt)) & 15) == 0;
+  // bulk copies want 16-byte boundaries: of the keys and of the payloads (the
+  // buffers in the scratch start on 256-byte ones)
+  a.use_bulk = ((((uintptr_t)keys) | (vw ? (uintptr_t)vals : 0)) & 15) == 0;
   a.sms = gprtcu_num_sms();
   if (small) return small_for(slot)(a, stream);
   return table_for(slot)[index](a, stream);

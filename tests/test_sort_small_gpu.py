@@ -44,3 +44,23 @@ def test_few_keys(cuda, kw, vw, n):
                                296 * 8192 + 1, (1 << 23) + 5])
 def test_default_shapes(cuda, kw, vw, n):
     _check(kw, vw, n, 0, 8 * kw if n < (1 << 21) else 30, n % 2 == 0, n)
+
+
+@pytest.mark.parametrize("n", [100, 8193, 20_001, 700_003])
+@pytest.mark.parametrize("key,value", [(4, 4), (4, 8), (8, 4), (8, 8)])
+@pytest.mark.parametrize("shift_k,shift_v", [(0, 1), (1, 0), (1, 1)])
+def test_buffers_off_16_byte_boundaries(cuda, n, key, value, shift_k, shift_v):
+    """Keys or payloads one element past an allocation's start: bulk copies
+    cannot take them."""
+    import torch
+    from gprt_b200 import api
+    k = np.random.default_rng(n).integers(0, 2 ** 12, n, dtype=np.uint64).astype(np.uint32 if key == 4 else np.uint64)
+    kd = torch.zeros(n + 1, dtype=torch.int32 if key == 4 else torch.int64, device="cuda")[shift_k:shift_k + n]
+    vd = torch.zeros(n + 1, dtype=torch.int32 if value == 4 else torch.int64, device="cuda")[shift_v:shift_v + n]
+    kd.copy_(torch.from_numpy(k.view(np.int32 if key == 4 else np.int64)))
+    vd.copy_(torch.arange(n))
+    assert kd.data_ptr() % 16 == key * shift_k and vd.data_ptr() % 16 == value * shift_v
+    api.sort(kd, vd)
+    order = np.argsort(k, kind="stable")
+    assert np.array_equal(kd.cpu().numpy().view(k.dtype), k[order])
+    assert np.array_equal(vd.cpu().numpy().astype(np.int64), order)
