@@ -578,6 +578,9 @@ __global__ void __launch_bounds__(WARPS * 32, (Pass8Cfg<K, V, WARPS, ITEMS, RANK
   using LB = LbWord<WIDE>;
   using SW = typename LB::T;
   constexpr int RADIX = C::RADIX, THREADS = C::THREADS, TILE = C::TILE, WK = C::WARP_KEYS;
+  // whether the last tile comes by bulk copies as far as it goes (at 1024 keys
+  // the threads' own loads are as fast)
+  constexpr bool PART = TILE > 1024;
   SortHeader *hdr = a.hdr;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // The pass's words, this thread's digit offset and (thread 0) the tile
@@ -623,14 +626,20 @@ __global__ void __launch_bounds__(WARPS * 32, (Pass8Cfg<K, V, WARPS, ITEMS, RANK
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
     fence_mbar_init();
-    // thread 0 knows the tile: its copies start before the block barrier
-    if (a.use_bulk && ((uint64_t)ticket + 1) * TILE <= a.n) {
-      const uint64_t ts = (uint64_t)ticket * TILE;
-      mbar_arrive_expect_tx(&bars[0], (uint32_t)C::KEY_BYTES);
-      bulk_g2s(s_keys, src_k + ts, (uint32_t)C::KEY_BYTES, &bars[0]);
-      if constexpr (C::HAS_V) {
-        mbar_arrive_expect_tx(&bars[1], (uint32_t)C::VAL_BYTES);
-        bulk_g2s(s_vals, src_v + ts, (uint32_t)C::VAL_BYTES, &bars[1]);
+    // thread 0 knows the tile: its copies start before the block barrier (the
+    // last tile's too, but for the end that is no multiple of 16 bytes: loaded
+    // by the threads, four fifths of a tile of 4096 u64 pairs took 4 us a pass;
+    // 540,001 pairs 141 -> 111 us)
+    const uint64_t ts = (uint64_t)ticket * TILE;
+    const uint32_t tn = PART ? (uint32_t)min((uint64_t)TILE, a.n - ts) : (ts + TILE <= a.n ? TILE : 0);
+    if (const uint32_t kb = tn * (uint32_t)sizeof(K) & ~15u; a.use_bulk && kb) {
+      mbar_arrive_expect_tx(&bars[0], kb);
+      bulk_g2s(s_keys, src_k + ts, kb, &bars[0]);
+    }
+    if constexpr (C::HAS_V) {
+      if (const uint32_t vb = tn * (uint32_t)sizeof(V) & ~15u; a.use_bulk && vb) {
+        mbar_arrive_expect_tx(&bars[1], vb);
+        bulk_g2s(s_vals, src_v + ts, vb, &bars[1]);
       }
     }
     // The tile that a CTA starting about pf_tiles tickets later will take:
@@ -647,29 +656,29 @@ __global__ void __launch_bounds__(WARPS * 32, (Pass8Cfg<K, V, WARPS, ITEMS, RANK
   const uint64_t tile_start = (uint64_t)tile * TILE;
   const uint32_t tile_n = (uint32_t)min((uint64_t)TILE, a.n - tile_start);
   const bool full = tile_n == TILE;
-  const bool bulk = a.use_bulk && full;
+  // what the copies above bring
+  const uint32_t bulk_k = a.use_bulk && (PART || full) ? (tile_n * (uint32_t)sizeof(K) & ~15u) / (uint32_t)sizeof(K) : 0u;
+  const uint32_t bulk_v =
+      a.use_bulk && C::HAS_V && (PART || full) ? (tile_n * (uint32_t)sizeof(V) & ~15u) / (uint32_t)sizeof(V) : 0u;
   {
     uint4 *t4 = reinterpret_cast<uint4 *>(s_cnt);  // counts and (RANK 2) masks are adjacent
     for (int i = tid; i < (int)((C::TBL_BYTES + C::MSK_BYTES) / 16); i += THREADS) t4[i] = make_uint4(0u, 0u, 0u, 0u);
   }
   for (int i = tid; i < RADIX; i += THREADS) status_next[(uint64_t)tile * RADIX + i] = 0;
-  if (!bulk) {
+  if (bulk_k < TILE) {
     // The last tile is padded with all-ones keys: they rank after every real
     // key within the top digit, so the real keys fill slots [0, tile_n).
-    for (int i = tid; i < TILE; i += THREADS) s_keys[i] = (uint32_t)i < tile_n ? src_k[tile_start + i] : ~(K)0;
+    for (uint32_t i = bulk_k + tid; i < TILE; i += THREADS) s_keys[i] = i < tile_n ? src_k[tile_start + i] : ~(K)0;
     if constexpr (C::HAS_V)
-      for (int i = tid; i < TILE; i += THREADS)
-        if ((uint32_t)i < tile_n) s_vals[i] = src_v[tile_start + i];
-  } else if (!mbar_wait(&bars[0], 0, mbar_budget_of(a.budget))) {
-    s_abort = 1;
+      for (uint32_t i = bulk_v + tid; i < tile_n; i += THREADS) s_vals[i] = src_v[tile_start + i];
   }
+  if (bulk_k && !mbar_wait(&bars[0], 0, mbar_budget_of(a.budget))) s_abort = 1;
   auto leave = [&]() {
     if (tid == 0) {
       record_error(&hdr->h, GPRTCU_ERR_TIMEOUT);
-      if (bulk) {
-        mbar_wait(&bars[0], 0, mbar_budget_of(a.budget));
-        if constexpr (C::HAS_V) mbar_wait(&bars[1], 0, mbar_budget_of(a.budget));
-      }
+      if (bulk_k) mbar_wait(&bars[0], 0, mbar_budget_of(a.budget));
+      if constexpr (C::HAS_V)
+        if (bulk_v) mbar_wait(&bars[1], 0, mbar_budget_of(a.budget));
     }
   };
   __syncthreads();
@@ -823,7 +832,7 @@ __global__ void __launch_bounds__(WARPS * 32, (Pass8Cfg<K, V, WARPS, ITEMS, RANK
     s_goff[tid] = ghist + excl - tstart;
   }
   if constexpr (C::HAS_V)
-    if (bulk && !mbar_wait(&bars[1], 0, mbar_budget_of(a.budget))) s_abort = 1;
+    if (bulk_v && !mbar_wait(&bars[1], 0, mbar_budget_of(a.budget))) s_abort = 1;
   __syncthreads();  // order complete; payload tile landed (s_abort visible)
   if (s_abort) {
     leave();

@@ -66,3 +66,22 @@ def test_sizes_around_the_lines(cuda, key, value):
         assert np.array_equal(kd.cpu().numpy().view(k.dtype), k[order])
         if value:
             assert np.array_equal(vd.cpu().numpy().astype(np.int64), order)
+
+
+def test_ragged_last_tile_time(cuda):
+    """A last tile that is nearly full costs what a full one does."""
+    import torch
+    from gprt_b200 import api
+    times = []
+    for n in (132 * 4096, 131 * 4096 + 3501):
+        k0 = torch.randint(-2 ** 63, 2 ** 63 - 1, (n,), generator=torch.Generator("cuda").manual_seed(1), device="cuda")
+        v0 = torch.arange(n, device="cuda")
+        k, v, scr = torch.empty_like(k0), torch.empty_like(v0), api.scratch(api.sort_scratch_size(n, 8, 8))
+
+        def run():
+            k.copy_(k0)
+            v.copy_(v0)
+            api.sort_with_config(k, v, (8, 4096, 8), scr=scr)
+
+        times.append(_us(run))
+    assert times[1] < 1.1 * times[0], times

@@ -64,3 +64,24 @@ def test_buffers_off_16_byte_boundaries(cuda, n, key, value, shift_k, shift_v):
     order = np.argsort(k, kind="stable")
     assert np.array_equal(kd.cpu().numpy().view(k.dtype), k[order])
     assert np.array_equal(vd.cpu().numpy().astype(np.int64), order)
+
+
+@pytest.mark.parametrize("key,value", TYPES)
+def test_last_tile_lengths(cuda, key, value):
+    """A last tile of every length modulo the 16 bytes that bulk copies move,
+    from one key up, at each tile size of the default shapes."""
+    import torch
+    from gprt_b200 import api
+    for tile in (1024, 2048, 4096, 6144, 8192):
+        for rest in (1, 2, 3, 4, 5, 7, 15, tile // 2 + 1, tile - 3, tile - 1, tile):
+            n = 3 * tile + rest
+            k = np.random.default_rng(rest).integers(0, 2 ** 16, n, dtype=np.uint64).astype(
+                np.uint32 if key == 4 else np.uint64)
+            k[-1] = np.iinfo(k.dtype).max  # as large as what fills the tile up
+            kd = torch.from_numpy(k.view(np.int32 if key == 4 else np.int64).copy()).cuda()
+            vd = None if not value else torch.arange(n, device="cuda", dtype=torch.int32 if value == 4 else torch.int64)
+            api.sort_with_config(kd, vd, (8, tile, 8))
+            order = np.argsort(k, kind="stable")
+            assert np.array_equal(kd.cpu().numpy().view(k.dtype), k[order]), n
+            if value:
+                assert np.array_equal(vd.cpu().numpy().astype(np.int64), order), n
