@@ -306,20 +306,23 @@ __device__ __forceinline__ bool warp_take(bool active, bool &drained, int lanes,
 
 // Grid of a persistent ray kernel (`ctas` CTAs of `warps` warps fit on an SM)
 // and the rays a warp holds at a time: all 32 lanes once there are rays for
-// kSpreadWarps warps per SM; fewer rays are spread over that many warps
+// `spread_warps` warps per SM; fewer rays are spread over that many warps
 // instead, at least four to each (a warp's time is that of its longest ray,
 // and lanes without a ray still run queued primitive tests).  4,099 rays on
 // 1,501 triangles at 32 / 16 / 8 / 4 / 2 / 1 rays per warp: 102 / 85 / 81 / 78
 // / 78 / 93 us.  8 / 12 / 16 / 24 warps per SM: any hit of 25,001 rays on 2,657
 // triangles 58.4 / 57.6 / 55.5 / 57.9 us, of 56,001 on 20,001 triangles 130 /
 // 130 / 131 / 137 us, of 40,001 on 4.2 M triangles 1,063 / 960 / 917 / 908 us.
+// Over instances 8, whose rays have more to share: 20,001 rays over 64
+// instances of 4 / 64 / 16 meshes 148 / 84 / 70 us with 8 warps per SM, 152 / 87
+// / 72 with 16.
 constexpr int kSpreadWarps = 16;
 struct RayGrid {
   int ctas, lanes;
 };
-static inline RayGrid ray_grid(uint64_t nrays, int ctas, int warps) {
+static inline RayGrid ray_grid(uint64_t nrays, int ctas, int warps, int spread_warps = kSpreadWarps) {
   const uint64_t fit = (uint64_t)gprtcu_num_sms() * ctas;
-  const uint64_t spread = (uint64_t)gprtcu_num_sms() * kSpreadWarps;
+  const uint64_t spread = (uint64_t)gprtcu_num_sms() * spread_warps;
   const uint64_t share = (nrays + spread - 1) / spread;
   const int lanes = share >= 32 ? 32 : (share < 4 ? 4 : (int)share);
   const uint64_t need = (nrays + (uint64_t)lanes * warps - 1) / ((uint64_t)lanes * warps);

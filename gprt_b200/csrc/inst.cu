@@ -137,7 +137,6 @@ constexpr int kInstShared = 10;  // stack entries in shared memory
 constexpr int kInstDepth = 128;  // 62 levels of each tree
 constexpr int kInstRefill = 4;
 constexpr int kInstSteps = 6;
-constexpr int kInstStepsLast = 12;
 constexpr int kInstFlush = 12;
 constexpr int kInstQueue = 96;  // a step queues at most 64
 constexpr int kInstCtas = 8;
@@ -195,10 +194,9 @@ __device__ __forceinline__ void inst_refine(const InstArgs &A, const InstRefineQ
 // comes once every lane still walking has a test queued (four at least): over
 // few instances a warp's last rays otherwise walk on with a stale culling
 // distance.  20,001 rays over 64 instances of 64 / 4 meshes, 400,001 triangles
-// together: 101 / 171 -> 87 / 152 us (92 / 163 in the plain walk); with 3,000
+// together: 101 / 171 -> 84 / 148 us (92 / 163 in the plain walk); with 3,000
 // instances as before; 115,001 rays over 200 instances of 4 meshes 367 -> 377 us
-// (422).  Six or eight tests at least: 99 / 91 us on the first.  12 instead of 6
-// node steps between two looks from then on: 5 % on these.
+// (422).  Six or eight tests at least: 99 / 91 us on the first.
 template <bool ANY, bool V8>
 __global__ void __launch_bounds__(kInstThreads, kInstCtas) k_trace_inst(const InstArgs A) {
   __shared__ float2 s_stack[kInstShared][kInstThreads];
@@ -333,7 +331,7 @@ __global__ void __launch_bounds__(kInstThreads, kInstCtas) k_trace_inst(const In
       continue;
     }
 #pragma unroll 1
-    for (int step = 0; step < (drained ? kInstStepsLast : kInstSteps); ++step) {
+    for (int step = 0; step < kInstSteps; ++step) {
       const bool on = W.node >= 0;
       float t0 = kNone, t1 = kNone;
       int r0 = 0, r1 = 0;
@@ -525,7 +523,7 @@ extern "C" GPRTCU_API gprtcuStatus gprtcuTraceInstances(const gprtcuLbvh *tlas, 
   ScratchHeader *hdr = (ScratchHeader *)scratch;
   unsigned long long *counter = reinterpret_cast<unsigned long long *>(&hdr->ticket[0]);
   GPRTCU_TRY(cudaMemsetAsync(scratch, 0, sizeof(ScratchHeader), stream));
-  const RayGrid g = ray_grid(numRays, kInstCtas, kInstWarps);
+  const RayGrid g = ray_grid(numRays, kInstCtas, kInstWarps, 8);
   InstArgs a;
   a.tnodes = (const Bvh2Node *)tlas->bvh2;
   a.tids = tlas->ids;
