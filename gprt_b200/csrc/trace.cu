@@ -124,8 +124,10 @@ __device__ __forceinline__ void finish_rays(const TraceArgs &A, RefineQueue &q, 
 // mesh and n its triangles.
 // Rays beyond the 151,552 that 148 SMs hold at once start as soon as this many
 // of a warp's lanes are idle: at 8 / 4 lanes 185,001 rays on 5,001 triangles
-// take 160 / 156 us.
+// take 160 / 156 us.  The rays of a batch are shorter: 77 M rays over 4,096
+// meshes at 4 / 8 / 16 lanes 33.6 / 32.4 / 33.3 ms.
 constexpr int kTraceRefill = 4;
+constexpr int kBatchRefill = 8;
 // One mesh whose nodes and leaves (112 bytes a triangle) pass some 560 MB: a
 // node that is not in L2 costs so much more from there on that rays which
 // start together are worth more than full lanes, since they meet in the upper
@@ -602,7 +604,7 @@ gprtcuStatus trace_launch(const gprtcuLbvh *bvh, const uint32_t *tri_off, const 
   };
   auto walk_batch = [&]() {
     auto launch = [&](auto kernel) { kernel<<<g.ctas, kTraceThreads, 0, stream>>>(a); };
-    constexpr int F = kTraceRefill;
+    constexpr int F = kBatchRefill;
     if (any) v8 ? launch(k_trace_any<true, true, F>) : launch(k_trace_any<true, false, F>);
     else v8 ? launch(k_trace_closest<true, true, F>) : launch(k_trace_closest<true, false, F>);
   };

@@ -207,7 +207,6 @@ template <typename PRIMS> struct UserArgs {
 
 constexpr int kUserThreads = 128;
 constexpr int kUserWarps = kUserThreads / 32;
-constexpr int kUserCtas = 7;
 constexpr int kUserShared = 12;  // stack entries in shared memory
 constexpr int kUserDepth = 64;
 constexpr int kUserRefill = 8;
@@ -334,12 +333,17 @@ __device__ __forceinline__ void user_odds(const UserArgs<PRIMS> &A, float2 odd) 
 // 12 stack entries in shared memory: 1.56 / 1.52 / 1.47 ms.)  With no more rays
 // to take, a flush comes as soon as the lanes still walking have a test each:
 // the culling distance lags less, which is worth more than full lanes then
-// (130,001 rays on 1,000,001 spheres 549 -> 481 us; 500 in the plain walk).  6 /
-// 7 / 8 CTAs per SM (80 / 72 / 64 registers, the last spilling 48 bytes): 1.47 /
-// 1.45 / 1.53 ms on the swept spheres above, 1.43 / 1.37 / 1.51 ms on as many
-// spheres; 10 / 14 node steps between two looks then 1.47 / 1.45 ms.
+// (130,001 rays on 1,000,001 spheres 549 -> 481 us; 500 in the plain walk).  7 /
+// 8 CTAs per SM (72 / 64 registers, the latter spilling some 30 bytes): 130,001
+// and 1,048,577 rays on a million spheres 481 / 507 us and 1.38 / 1.43 ms, on a
+// million swept spheres 461 / 478 us and 1.48 / 1.45 ms, 4.2 M rays on 4.2 M
+// swept spheres 4.82 / 4.55 ms: spheres run 7, swept spheres, which wait more on
+// memory, 8.  6 CTAs: 1.43 ms on the million spheres.  10 / 14 node steps between
+// two looks 1.47 / 1.45 ms on the million swept spheres.
+template <typename PRIMS> constexpr int kUserCtas = 7;
+template <> constexpr int kUserCtas<LssPrims> = 8;
 template <typename PRIMS, bool V8>
-__global__ void __launch_bounds__(kUserThreads, kUserCtas) k_user_closest(const UserArgs<PRIMS> A) {
+__global__ void __launch_bounds__(kUserThreads, kUserCtas<PRIMS>) k_user_closest(const UserArgs<PRIMS> A) {
   __shared__ float2 s_stack[kUserShared][kUserThreads];
   __shared__ uint32_t s_qslot[kUserWarps][kUserQueue];
   __shared__ uint8_t s_qlane[kUserWarps][kUserQueue];
@@ -721,7 +725,7 @@ gprtcuStatus trace_user(const gprtcuLbvh *bvh, PRIMS prims, const float *rays, u
   // 50,001 269 / 250 / 272, 200,001 400 / 409 / 378; 10,001 swept spheres 77 / 81 /
   // 85, 50,001 186 / 172 / 187, 1,000,001 514 / 519 / 474.
   const RayGrid few = any ? RayGrid{0, 0} : pool_grid(nrays, bvh->numPrims <= 100000 ? 16 : 12);
-  const RayGrid g = few.lanes ? few : ray_grid(nrays, any ? kUserAnyCtas : kUserCtas, kUserWarps);
+  const RayGrid g = few.lanes ? few : ray_grid(nrays, any ? kUserAnyCtas : kUserCtas<PRIMS>, kUserWarps);
   UserArgs<PRIMS> a{(const Bvh2Node *)bvh->bvh2, bvh->ids, bvh->numPrims, bvh->rootBox, prims, exit_test != 0,
                     (const float4 *)rays, nrays, g.lanes, (Hit *)hits, u, counter, &hdr->status};
   auto launch = [&](auto kernel, int threads) { kernel<<<g.ctas, threads, 0, stream>>>(a); };
