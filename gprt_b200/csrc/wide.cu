@@ -5,7 +5,7 @@
 // ("Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide
 // BVHs"), written here for this build.
 //
-// Node (80 bytes, five 16-byte loads):
+// Node (80 bytes: five 16-byte words, read in three loads, see wide_word):
 //   p.xyz      fp32 origin = min corner of the children's union box
 //   e.xyz      scale exponents + 127 in a byte each, scale s = 2^e per axis,
 //              chosen (in FP64) as the smallest power of two with 255 * s >=
@@ -17,10 +17,12 @@
 //              leaf children
 //   qlo/qhi    per axis, per child: floor((lo - p) / s), ceil((hi - p) / s);
 //              an empty slot holds the inverted box qlo 255, qhi 0
-// Decoding uses round-down (lo) and round-up (hi) FMAs, so every decoded box
-// contains its exact fp32 child box; a ray therefore never misses a child the
-// binary traversal would enter, and intersection is the same FP32 watertight
-// test, giving the same hits.  A node is 80 bytes for up to eight children
+// Traversal moves a plane's offset down (near planes) or up (far planes) with
+// directed rounding and decodes it by one FMA that rounds to nearest, off by at
+// most 2^-24 of its own result, which the box test's widening by 2^-18 covers:
+// every decoded interval contains the exact child box's, a ray never misses a
+// child that the binary traversal would enter, and intersection is the same
+// FP32 watertight test, giving the same hits.  A node is 80 bytes for up to eight children
 // against 64 bytes for two in the binary layout.
 #include "common.cuh"
 #include "lbvh.cuh"
@@ -65,8 +67,8 @@ struct WorkItem {
 // index is its queue slot), LEAF the next free wide leaf slot, TICKET the
 // level kernel's CTA done-counter, EPOCH and NEXT (polled, so in a line of
 // their own) the levels that the last launch has finished and TAIL after the
-// latest of them.
-enum { C_LO = 0, C_HI = 1, C_TAIL = 2, C_LEAF = 3, C_TICKET = 4, C_EPOCH = 32, C_NEXT = 33 };
+// latest of them, MESHES the number of roots.
+enum { C_LO = 0, C_HI = 1, C_TAIL = 2, C_LEAF = 3, C_TICKET = 4, C_MESHES = 5, C_EPOCH = 32, C_NEXT = 33 };
 
 // Levels a collapse runs: a binary node splits its keys at the highest
 // differing bit of (30-bit code, 30-bit index), so binary and therefore wide
@@ -106,6 +108,7 @@ __global__ void k_wide_init(const uint32_t *tri_off, uint32_t meshes, uint32_t n
     counters[C_TAIL] = meshes;
     counters[C_LEAF] = 0;
     counters[C_TICKET] = 0;
+    counters[C_MESHES] = meshes;
   }
 }
 
@@ -123,8 +126,10 @@ __global__ void k_wide_init(const uint32_t *tri_off, uint32_t meshes, uint32_t n
 // from level to level by itself, a hardware barrier between them, while a level
 // has at most `most` items.  kWideRestForm takes whatever levels are left: all
 // its CTAs are on the GPU at once (a cooperative launch) and wait for one
-// another after each level, `most` polls at most, after which the call's
-// status is GPRTCU_ERR_TIMEOUT.  The eight candidate children stay in registers
+// another after each level, `most` polls at most; a CTA whose wait runs out
+// sets the call's status to GPRTCU_ERR_TIMEOUT, empties every root, since nodes
+// below may not have been written, and leaves (so then do the others, and the
+// last of them has emptied the roots after all that was written).  The eight candidate children stay in registers
 // (unrolled loops, predicated updates) and quantising multiplies by the exact
 // power of two 2^-e instead of dividing by 2^e: on 67M triangles in 16,384
 // meshes the collapse went from 10.96 ms (local-memory arrays, FP64
@@ -336,7 +341,16 @@ __global__ void __launch_bounds__(128, FORM == kWideClusterForm ? 1 : 7) k_wide_
       }
       __syncthreads();
       const uint32_t tail = s_next;
-      if (tail <= hi) break;  // no items left (or the wait ran out)
+      if (tail == 0)  // the wait ran out
+        for (uint32_t m = threadIdx.x; m < counters[C_MESHES]; m += blockDim.x) {
+          uint4 *op = reinterpret_cast<uint4 *>(wnodes) + 5 * (size_t)(m & ~1u);
+          op[wide_word(m, 0)] = make_uint4(0u, 0u, 0u, 0u);
+          op[wide_word(m, 1)] = make_uint4(0u, 0u, ~0u, ~0u);
+          op[wide_word(m, 2)] = make_uint4(~0u, ~0u, ~0u, ~0u);
+          op[wide_word(m, 3)] = make_uint4(~0u, ~0u, 0u, 0u);
+          op[wide_word(m, 4)] = make_uint4(0u, 0u, 0u, 0u);
+        }
+      if (tail <= hi) break;  // no items left
       lo = hi;
       hi = tail;
     }

@@ -412,6 +412,9 @@ GPRTCU_API gprtcuStatus gprtcuBatchTrace(const gprtcuLbvh *bvh, const uint32_t *
  *   roots     uint32[numMeshes]: root node of each mesh
  *   numNodes  optional device uint32: node count written by the build
  * triOffsets / rayOffsets: NULL (one mesh) or device uint32[numMeshes+1].
+ * The collapse waits (bounded) for its own thread blocks; should a wait run
+ * out, its scratch's status is GPRTCU_ERR_TIMEOUT and every root is left without
+ * children.
  * ------------------------------------------------------------------------ */
 typedef struct {
   void *nodes;
@@ -455,8 +458,9 @@ GPRTCU_API gprtcuStatus gprtcuGenRays(uint64_t numRays, uint64_t seed, const uin
  * Test hooks (fault injection without a GPU fault).  Process-wide settings
  * read at launch time by the kernels that wait.  No counterpart in the
  * reference, whose waits happen inside the Vulkan driver.
- * gprtcuDebugSetSpinBudget: polls a look-back wait (scan, sort) or a refit's
- *   wait for its sibling makes before it records GPRTCU_ERR_TIMEOUT (0
+ * gprtcuDebugSetSpinBudget: polls a look-back wait (scan, sort), a refit's wait
+ *   for its sibling or a collapse's for its blocks makes before it records
+ *   GPRTCU_ERR_TIMEOUT (0
  *   restores the default, 2^22); the mbarrier waits of the TMA-staged kernels
  *   get 16 polls for each of these.  The refit's budget is set on the current
  *   device.

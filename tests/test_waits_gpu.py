@@ -228,3 +228,42 @@ def test_compat_sort_with_caller_scratch_reports_device_error_at_map(hooks):
             L.gprtBufferDestroy(b)
         L.gprtContextDestroy(ctx)
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("meshes", [1, 300])
+def test_collapse_block_wait_timeout_is_reported_and_stays_in_bounds(hooks, meshes):
+    # The launch that takes a tree's last levels waits for its own blocks
+    # after each; with a budget of one poll the first to finish a level gives
+    # up.  The status says so, and every root is left empty, so a trace reads
+    # no node that was not written.  (300 meshes: all levels by that launch,
+    # as on a device without clusters of eight blocks.)
+    import torch
+    from gprt_b200 import api, scenes
+    rng = np.random.default_rng(3)
+    n = 300_000
+    k = 2.0**(-25 * rng.random((n, 1)))
+    pos = ((rng.random((n, 3)) * k)[:, None, :] + rng.normal(0, 0.01, (n, 3, 3)) * k[:, None, :])
+    p = torch.from_numpy(pos.reshape(-1, 3).astype(np.float32)).cuda()
+    t = torch.arange(3 * n, dtype=torch.int32, device="cuda").view(n, 3)
+    rays = torch.from_numpy(scenes.rays(3000, seed=4)).cuda()
+    roff = torch.from_numpy(np.linspace(0, 3000, meshes + 1).astype(np.int32)).cuda()
+    if meshes == 1:
+        b = api.lbvh_build_triangles(p, t)
+    else:
+        b = api.batch_build_triangles(p, t, api.BatchLbvh(np.linspace(0, n, meshes + 1).astype(np.int64)))
+        hooks.gprtcuDebugMaxCluster(1)
+    w = api.WideBvh(n, meshes)
+    torch.cuda.synchronize()
+    hooks.gprtcuDebugSetSpinBudget(1)
+    api.wide_build(b, wide=w)
+    torch.cuda.synchronize()
+    hooks.gprtcuDebugSetSpinBudget(0)
+    hooks.gprtcuDebugMaxCluster(0)
+    assert api.scratch_status(w.scratch) == TIMEOUT
+    for anyhit in (False, True):
+        assert bool((api.wide_trace(w, rays, roff, anyhit=anyhit)[:, 0] == -1).all())
+    api.wide_build(b, wide=w)
+    assert api.scratch_status(w.scratch) == 0
+    exp = api.trace(b, rays) if meshes == 1 else api.batch_trace(b, rays, roff)
+    assert torch.equal(api.wide_trace(w, rays, roff), exp)
+    assert bool((exp[:, 0] != -1).any())
