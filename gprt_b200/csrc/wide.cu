@@ -3,7 +3,7 @@
 // the reference (its traversal is Vulkan ray-tracing hardware); the node
 // format follows the compressed-wide-BVH idea of Ylitie, Karras, Laine 2017
 // ("Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide
-// BVHs"), written here for this build.
+// BVHs"), written here for this library.
 //
 // Node (80 bytes: five 16-byte words, read in three loads, see wide_word):
 //   p.xyz      fp32 origin = min corner of the children's union box
