@@ -174,9 +174,19 @@ __device__ __forceinline__ bool take_rays(const TraceArgs &A, bool active, bool 
 // on 100,001 triangles: votes at every / 2nd / 4th / 8th visit 1,564 / 1,553 /
 // 1,540 / 1,538 us; then nodes alone on the stack 1,470, every 12th visit 1,464
 // us.  10 CTAs per SM spill: 1,547 us.  Stack entries in shared memory 12 / 6 /
-// 3: 1,461 / 1,474 / 1,547 us.
+// 3: 1,461 / 1,474 / 1,547 us.  One pass over the test for the first leaf of a
+// step, whichever child it is: 8,001 rays on 100,001 triangles 168 -> 164 us.
+//
+// A grid of at most kAnyFewCtas per SM (113,664 rays on 148 SMs) asks for no
+// more shared memory than those need (kAnyCarveout per cent of what an SM can
+// give), which leaves L1 more: its walks wait for loads.  56,001 / 115,001 rays
+// on 2,657 triangles 65.4 -> 60.8 us, 80.7 -> 74 us.  28 / 12 per cent: 62.6 / 73
+// us, the latter leaving room for three CTAs.  Above, all 8 are worth more:
+// 1,000,001 rays on 735 triangles 240 us, 256 with the carveout.
 constexpr int kAnySteps = 12;
 constexpr int kAnyCtas = 8;
+constexpr int kAnyFewCtas = 6;
+constexpr int kAnyCarveout = 20;
 constexpr int kAnyShared = 12;  // stack entries in shared memory
 template <bool BATCHED, bool V8, int REFILL>
 __global__ void __launch_bounds__(kTraceThreads, kAnyCtas) k_trace_any(const TraceArgs A) {
@@ -254,8 +264,11 @@ __global__ void __launch_bounds__(kTraceThreads, kAnyCtas) k_trace_any(const Tra
         const ChildPairs c0 = load_child<V8>(&nd->c[0]), c1 = load_child<V8>(&nd->c[1]);
         float t0, t1;
         const bool h0 = child_hit(c0, P, bt, t0), h1 = child_hit(c1, P, bt, t1);
-        if (h0 && c0.ref < 0) leaf_test(base_leaf + (uint32_t)~c0.ref);
-        if (h1 && c1.ref < 0 && t1 <= bt) leaf_test(base_leaf + (uint32_t)~c1.ref);
+        const bool l0 = h0 && c0.ref < 0, l1 = h1 && c1.ref < 0;
+        if (l0 || l1) {  // a lane's first leaf shares one pass over the test, whichever child it is
+          leaf_test(base_leaf + (uint32_t)~(l0 ? c0.ref : c1.ref));
+          if (l0 && l1 && t1 <= bt) leaf_test(base_leaf + (uint32_t)~c1.ref);
+        }
         const bool in0 = h0 && c0.ref >= 0, in1 = h1 && c1.ref >= 0;
         const bool first = in0 && !(in1 && t1 < t0);  // the nearer child, child 0 on ties
         if (best != kMiss) {
@@ -596,16 +609,28 @@ gprtcuStatus trace_launch(const gprtcuLbvh *bvh, const uint32_t *tri_off, const 
   a.counter = counter;
   a.err = &hdr->status;
   const bool v8 = ((uintptr_t)bvh->bvh2 & 31) == 0;
+  auto launch_any = [&](auto kernel) {
+    cudaLaunchAttribute carveout;
+    carveout.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    carveout.val.sharedMemCarveout = kAnyCarveout;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(g.ctas);
+    cfg.blockDim = dim3(kTraceThreads);
+    cfg.stream = stream;
+    cfg.attrs = &carveout;
+    cfg.numAttrs = g.ctas <= gprtcu_num_sms() * kAnyFewCtas ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, a);  // its error is taken up below
+  };
   auto walk = [&](auto refill) {
     constexpr int F = decltype(refill)::value;
     auto launch = [&](auto kernel) { kernel<<<g.ctas, kTraceThreads, 0, stream>>>(a); };
-    if (any) v8 ? launch(k_trace_any<false, true, F>) : launch(k_trace_any<false, false, F>);
+    if (any) v8 ? launch_any(k_trace_any<false, true, F>) : launch_any(k_trace_any<false, false, F>);
     else v8 ? launch(k_trace_closest<false, true, F>) : launch(k_trace_closest<false, false, F>);
   };
   auto walk_batch = [&]() {
     auto launch = [&](auto kernel) { kernel<<<g.ctas, kTraceThreads, 0, stream>>>(a); };
     constexpr int F = kBatchRefill;
-    if (any) v8 ? launch(k_trace_any<true, true, F>) : launch(k_trace_any<true, false, F>);
+    if (any) v8 ? launch_any(k_trace_any<true, true, F>) : launch_any(k_trace_any<true, false, F>);
     else v8 ? launch(k_trace_closest<true, true, F>) : launch(k_trace_closest<true, false, F>);
   };
   // The pool (closest hit) while it is the faster form: up to 9/6 chunks per
