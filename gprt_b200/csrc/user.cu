@@ -502,13 +502,15 @@ __global__ void __launch_bounds__(kUserThreads, kUserCtas<PRIMS>) k_user_closest
 // nodes alone (the closest-hit kernel with its tests at once kept them in
 // shared memory, 17 KB a CTA): 30,001 / 1,000,001 rays on 1,000,001 swept
 // spheres 344 / 1,697 -> 317 / 1,504 us, 150,001 rays on 10,001 spheres 149 ->
-// 122 us.  Steps between two votes 12 / 12 and 48 once there are no more
+// 122 us.  Closest hit in the same form (trace_user: few primitives) culls by
+// the best distance when a node is visited, in the order of user_odd, so a hit
+// at a distance that is no number needs no second walk.  Steps between two votes 12 / 12 and 48 once there are no more
 // rays to take: 20,001 rays on 1,001 spheres 29 / 33 us.
 constexpr int kUserAnyCtas = 8;
 constexpr int kUserAnyShared = 8;  // stack entries (nodes alone: nothing is culled by distance) in shared memory
 constexpr int kUserAnySteps = 12;
-template <typename PRIMS, bool V8>
-__global__ void __launch_bounds__(kUserThreads, kUserAnyCtas) k_user_any(const UserArgs<PRIMS> A) {
+template <typename PRIMS, bool ANY, bool V8>
+__global__ void __launch_bounds__(kUserThreads, kUserAnyCtas) k_user_lane(const UserArgs<PRIMS> A) {
   __shared__ int s_stack[kUserAnyShared][kUserThreads];
   bool active = false, drained = false;
   uint64_t r = 0;
@@ -577,9 +579,9 @@ __global__ void __launch_bounds__(kUserThreads, kUserAnyCtas) k_user_any(const U
         const bool h0 = child_hit(c0, P, bt, t0), h1 = child_hit(c1, P, bt, t1);
         if (h0 && c0.ref < 0) test((uint32_t)~c0.ref);
         if (h1 && c1.ref < 0 && t1 <= bt) test((uint32_t)~c1.ref);
-        const bool in0 = h0 && c0.ref >= 0, in1 = h1 && c1.ref >= 0;
+        const bool in0 = h0 && c0.ref >= 0, in1 = h1 && c1.ref >= 0 && (ANY || t1 <= bt);
         const bool first = in0 && !(in1 && t1 < t0);  // the nearer child, child 0 on ties
-        if (best != kMiss) {
+        if (ANY ? best != kMiss : bt != bt) {  // a hit at a distance that is no number is a ray's last
           node = -1;
         } else if (in0 || in1) {
           if (in0 && in1) {
@@ -723,14 +725,30 @@ gprtcuStatus trace_user(const gprtcuLbvh *bvh, PRIMS prims, const float *rays, u
   // on 148 SMs, and 16/6, 151,552 rays, for up to 100,000 primitives.  150,001
   // rays, plain walk / pool / lane per ray: 10,001 spheres 144 / 143 / 153 us,
   // 50,001 269 / 250 / 272, 200,001 400 / 409 / 378; 10,001 swept spheres 77 / 81 /
-  // 85, 50,001 186 / 172 / 187, 1,000,001 514 / 519 / 474.
-  const RayGrid few = any ? RayGrid{0, 0} : pool_grid(nrays, bvh->numPrims <= 100000 ? 16 : 12);
-  const RayGrid g = few.lanes ? few : ray_grid(nrays, any ? kUserAnyCtas : kUserCtas<PRIMS>, kUserWarps);
+  // 85, 50,001 186 / 172 / 187, 1,000,001 514 / 519 / 474.  Below
+  // 16,384 primitives, whose walks are short, it ends at 9/6, 85,248 rays (70,001
+  // on 10,001 swept spheres pool / k_user_lane 50.8 / 54.9 us), below 8,192 at
+  // 6/6.  From there up to one ray per lane that fits, below 2,048 for any
+  // number, the tests run where they are met (k_user_lane): where the primitives are apart a queue
+  // costs more than its full lanes give, and where they overlap that is still
+  // the faster of this and a plain walk.  Plain walk / what it was / now:
+  // 113,001 rays on 1,001 / 5,001 spheres 45.1 / 51.2 / 38.9 us, 84.4 / 86.9 / 73.9;
+  // on as many swept spheres 26.8 / 29.2 / 26.5, 49.5 / 49.4 / 45.4; 150,001 on
+  // 10,001 of them 77.5 / 81.7 / 69.3; 1,000,001 rays on 101 swept spheres 33.5 / 58.8 / 34.2, on 101 wide ones that overlap 883 /
+  // 650 / 759.  From 2,048 on the queue is the faster form again with more
+  // rays: 1,000,001 on 5,001 spheres that overlap 669 / 435 / 623.
+  const uint32_t n = bvh->numPrims;
+  const RayGrid few =
+      any ? RayGrid{0, 0} : pool_grid(nrays, n < 8192 ? 6 : n < 16384 ? 9 : n <= 100000 ? 16 : 12);
+  const bool lane = any || n < 2048 ||
+                    (n < 16384 && nrays <= (uint64_t)gprtcu_num_sms() * kUserAnyCtas * kUserThreads);
+  const RayGrid g = few.lanes ? few : ray_grid(nrays, lane ? kUserAnyCtas : kUserCtas<PRIMS>, kUserWarps);
   UserArgs<PRIMS> a{(const Bvh2Node *)bvh->bvh2, bvh->ids, bvh->numPrims, bvh->rootBox, prims, exit_test != 0,
                     (const float4 *)rays, nrays, g.lanes, (Hit *)hits, u, counter, &hdr->status};
   auto launch = [&](auto kernel, int threads) { kernel<<<g.ctas, threads, 0, stream>>>(a); };
-  if (any) v8 ? launch(k_user_any<PRIMS, true>, kUserThreads) : launch(k_user_any<PRIMS, false>, kUserThreads);
+  if (any) v8 ? launch(k_user_lane<PRIMS, true, true>, kUserThreads) : launch(k_user_lane<PRIMS, true, false>, kUserThreads);
   else if (few.lanes) v8 ? launch(k_user_pool<PRIMS, true>, kPoolThreads) : launch(k_user_pool<PRIMS, false>, kPoolThreads);
+  else if (lane) v8 ? launch(k_user_lane<PRIMS, false, true>, kUserThreads) : launch(k_user_lane<PRIMS, false, false>, kUserThreads);
   else v8 ? launch(k_user_closest<PRIMS, true>, kUserThreads) : launch(k_user_closest<PRIMS, false>, kUserThreads);
   GPRTCU_TRY(cudaGetLastError());
   return GPRTCU_OK;

@@ -120,3 +120,76 @@ def test_no_step_at_the_line(cuda):
 
     below, above = us(rays[:a]), us(rays)
     assert above < slack * below and below < slack * above, (below, above)
+
+
+def _scene(kind, n, reach=0.0):
+    """n primitives apart from each other (as strands), or within `reach`."""
+    rng = np.random.default_rng(n)
+    v = np.concatenate([rng.random((n + 1, 3)), rng.uniform(0.0005, 0.002 + reach, (n + 1, 1))], 1).astype(np.float32)
+    v[1::2, :3] = v[:-1:2, :3][:len(v[1::2])] + rng.normal(0, 0.004 + reach, (len(v[1::2]), 3)).astype(np.float32)
+    idx = np.stack([np.arange(n) & ~1, (np.arange(n) & ~1) + 1], 1).astype(np.uint32) % (n + 1)
+    return (v[:n] if kind == "spheres" else v), idx
+
+
+def _runner(kind, v, idx):
+    import torch
+    from gprt_b200 import api
+    vt, it = torch.from_numpy(v).cuda(), torch.from_numpy(idx.view(np.int32)).cuda()
+    if kind == "spheres":
+        b = api.lbvh_build_boxes(api.sphere_bounds(vt))
+        return lambda r, **k: api.trace_spheres(b, vt, r, **k)
+    b = api.lbvh_build_boxes(api.lss_bounds(vt, it))
+    return lambda r, **k: api.trace_lss(b, vt, it, r, **k)
+
+
+@pytest.mark.parametrize("reach", [0.0, 0.1])
+@pytest.mark.parametrize("n", [1, 2, 2047, 2048, 8191, 8192, 16383])
+@pytest.mark.parametrize("kind", ["spheres", "lss"])
+def test_few_prims_lines(cuda, kind, n, reach):
+    """Few primitives: the same hits and u on both sides of each ray count
+    where the form changes, exit hits too, and the oracle's primitives."""
+    import torch
+    v, idx = _scene(kind, n, reach)
+    run = _runner(kind, v, idx)
+    lines = [_line(6), _line(9), _sms() * 8 * 128]
+    m = lines[-1] + 1
+    rays_h = scenes.rays(m, seed=n)
+    rays_h[::97, 7] = np.nan
+    rays_h[5::97, 3] = -1.0
+    rays = torch.from_numpy(rays_h).cuda()
+    for exit_test in (False, True):
+        u = torch.zeros(m, device="cuda")
+        full = _bits(run(rays, u=u, exit_test=exit_test)).copy()
+        for k in (1, 4099, lines[0], lines[0] + 1, lines[1], lines[1] + 1, lines[2]):
+            w = torch.zeros(k, device="cuda")
+            assert np.array_equal(_bits(run(rays[:k], u=w, exit_test=exit_test)), full[:k])
+            assert torch.equal(w.view(torch.int32), u[:k].view(torch.int32))
+        if not exit_test:
+            ok = np.arange(m - 300, m)[~np.isnan(rays_h[-300:, 7])]
+            e = oracle.trace_user_brute(0 if kind == "spheres" else 1, v, rays_h[ok],
+                                        *(() if kind == "spheres" else (idx,)))
+            assert np.array_equal(full[ok, 0], e["prim"])
+
+
+@pytest.mark.parametrize("kind,n,m", [("spheres", 1001, 130001), ("lss", 1001, 130001), ("lss", 101, 1000001)])
+def test_few_prims_take_no_longer_than_any_hit(cuda, kind, n, m):
+    """Few primitives that lie apart, which most rays miss: a closest hit has
+    little more to do than an any hit."""
+    import torch
+    from gprt_b200 import api
+    run, rays = _runner(kind, *_scene(kind, n)), api.gen_rays(m, seed=5)
+    hits, scr = torch.empty((m, 2), dtype=torch.int32, device="cuda"), api.scratch(256)
+
+    def us(any_hit):
+        times = []
+        for _ in range(9):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            for _ in range(20):
+                run(rays, hits=hits, scr=scr, anyhit=any_hit)
+            e[1].record()
+            e[1].synchronize()
+            times.append(50.0 * e[0].elapsed_time(e[1]))
+        return sorted(times[2:])[3]
+
+    assert us(False) < 1.15 * us(True)
