@@ -496,18 +496,19 @@ __global__ void __launch_bounds__(kUserThreads, kUserCtas<PRIMS>) k_user_closest
   user_odds(A, odd);
 }
 
-// Any hit: the primitives of the leaf children that a step meets are tested
+// Any hit (ANY): the primitives of the leaf children that a step meets are tested
 // at once, child 0 first, and the first step with a hit ends the ray, as the
 // any-hit walk over triangles does.  Ray and hit in registers and a stack of
 // nodes alone (the closest-hit kernel with its tests at once kept them in
 // shared memory, 17 KB a CTA): 30,001 / 1,000,001 rays on 1,000,001 swept
 // spheres 344 / 1,697 -> 317 / 1,504 us, 150,001 rays on 10,001 spheres 149 ->
-// 122 us.  Closest hit in the same form (trace_user: few primitives) culls by
-// the best distance when a node is visited, in the order of user_odd, so a hit
-// at a distance that is no number needs no second walk.  Steps between two votes 12 / 12 and 48 once there are no more
-// rays to take: 20,001 rays on 1,001 spheres 29 / 33 us.
+// 122 us.  Steps between two votes 12 / 12 and 48 once there are no more rays to
+// take: 20,001 rays on 1,001 spheres 29 / 33 us.  Closest hit in the same form
+// (few primitives: trace_user) culls by the best distance when it visits a
+// node, not when it takes it off the stack, and keeps to the order of
+// user_odd, so a hit at a distance that is no number needs no second walk.
 constexpr int kUserAnyCtas = 8;
-constexpr int kUserAnyShared = 8;  // stack entries (nodes alone: nothing is culled by distance) in shared memory
+constexpr int kUserAnyShared = 8;  // stack entries (nodes alone) in shared memory
 constexpr int kUserAnySteps = 12;
 template <typename PRIMS, bool ANY, bool V8>
 __global__ void __launch_bounds__(kUserThreads, kUserAnyCtas) k_user_lane(const UserArgs<PRIMS> A) {
@@ -726,17 +727,18 @@ gprtcuStatus trace_user(const gprtcuLbvh *bvh, PRIMS prims, const float *rays, u
   // rays, plain walk / pool / lane per ray: 10,001 spheres 144 / 143 / 153 us,
   // 50,001 269 / 250 / 272, 200,001 400 / 409 / 378; 10,001 swept spheres 77 / 81 /
   // 85, 50,001 186 / 172 / 187, 1,000,001 514 / 519 / 474.  Below
-  // 16,384 primitives, whose walks are short, it ends at 9/6, 85,248 rays (70,001
-  // on 10,001 swept spheres pool / k_user_lane 50.8 / 54.9 us), below 8,192 at
-  // 6/6.  From there up to one ray per lane that fits, below 2,048 for any
-  // number, the tests run where they are met (k_user_lane): where the primitives are apart a queue
-  // costs more than its full lanes give, and where they overlap that is still
-  // the faster of this and a plain walk.  Plain walk / what it was / now:
-  // 113,001 rays on 1,001 / 5,001 spheres 45.1 / 51.2 / 38.9 us, 84.4 / 86.9 / 73.9;
-  // on as many swept spheres 26.8 / 29.2 / 26.5, 49.5 / 49.4 / 45.4; 150,001 on
-  // 10,001 of them 77.5 / 81.7 / 69.3; 1,000,001 rays on 101 swept spheres 33.5 / 58.8 / 34.2, on 101 wide ones that overlap 883 /
-  // 650 / 759.  From 2,048 on the queue is the faster form again with more
-  // rays: 1,000,001 on 5,001 spheres that overlap 669 / 435 / 623.
+  // 16,384 primitives, whose walks are short, it ends at 9/6, 85,248 rays
+  // (70,001 on 10,001 swept spheres pool / k_user_lane 50.8 / 54.9 us), below
+  // 8,192 at 6/6.  From there up to one ray per lane that fits, and below 2,048
+  // for any number, the tests run where they are met (k_user_lane): where
+  // primitives lie apart a queue costs more than its full lanes give, and
+  // where they overlap this is still faster than a plain walk.  Plain walk /
+  // pool or queue / k_user_lane: 113,001 rays on 1,001 spheres 45.1 / 51.2 /
+  // 38.9 us, on 5,001 84.4 / 86.9 / 73.9, on as many swept spheres 26.8 / 29.2 /
+  // 26.5 and 49.5 / 49.4 / 45.4; 150,001 on 10,001 of them 77.5 / 81.7 / 69.3;
+  // 1,000,001 on 101 of them 33.5 / 58.8 / 34.2, on 101 wide ones that overlap
+  // 883 / 650 / 759.  From 2,048 on, more rays find the queue faster or level:
+  // 1,000,001 on 5,001 spheres that overlap 669 / 435 / 623.
   const uint32_t n = bvh->numPrims;
   const RayGrid few =
       any ? RayGrid{0, 0} : pool_grid(nrays, n < 8192 ? 6 : n < 16384 ? 9 : n <= 100000 ? 16 : 12);
